@@ -83,15 +83,20 @@ __device__ __forceinline__ void storeCon(const StateP& s, long long c, const dou
 // pressure at rest, its faces carry no residual flux. side 1: WindBC (apps/wind.F90:224-319): the ghost is
 // the wind blended with an outflow copy of the last active cell (at least MinMach = 1 fast speed outward), its
 // faces the wind's flux blended with the last active face's.
-__global__ void k_bc_ionwind(Lay L, Par p, GridP g, StateP s, int side) {
+// blockIdx.y: 0 the inner side; 1 the cells and 2 + d the d-faces of the outer side, whose wind weights (an acos
+// and an exp each) are the work: the inner side's launch and then four weights in one thread took 5.0 + 20.0 us at
+// 96x96x128 (4.2 + 16.1 us at 48x42x64), now 18.4 us (8.7 us) for both sides.
+__global__ void k_bc_ionwind(Lay L, Par p, GridP g, StateP s) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int nG = L.nG, nj = L.Nj + 1;
     if (t >= (long long)nG * nj * (L.Nk + 1)) return;
+    const int part = blockIdx.y;
+    if (p.bc[part == 0 ? 0 : 1] != (part == 0 ? BC_ION : BC_WIND)) return;
     const int n = 1 + (int)(t % nG);
     const long long row = t / nG;
     const int j = (int)(row % nj), k = (int)(row / nj);
     const bool cell = (j < L.Nj) && (k < L.Nk);
-    if (side == 0) {
+    if (part == 0) {
         const int ig = L.is() - n, ip = L.is() + n - 1;
         if (cell) {
             int jp, kp;
@@ -111,7 +116,8 @@ __global__ void k_bc_ionwind(Lay L, Par p, GridP g, StateP s, int side) {
     }
     const MsphPar& m = p.msph;
     const int ip = L.ie(), ig = L.ie() + n;
-    if (cell) {
+    if (part == 1) {
+        if (!cell) return;
         const long long c = L.at(ig, j, k);
         double xcc[3] = {g.xyzcc[0][c], g.xyzcc[1][c], g.xyzcc[2][c]};
         double wSW = wgtWind(m, xcc), wMHD = 1.0 - wSW;
@@ -139,8 +145,8 @@ __global__ void k_bc_ionwind(Lay L, Par p, GridP g, StateP s, int side) {
         for (int v = 0; v < 5; ++v) gW[v] = wSW * gW_sw[v] + wMHD * gW_in[v];
         cellP2C(p, gW, gCon);
         storeCon(s, c, gCon);
-    }
-    for (int d = 0; d < 3; ++d) {
+    } else {
+        const int d = part - 2;
         const int fi = d == 0 ? ig + 1 : ig, si = d == 0 ? ip + 1 : ip;
         const long long f = L.at(fi, j, k);
         double xf[3] = {g.xfc[d][0][f], g.xfc[d][1][f], g.xfc[d][2][f]};
@@ -204,9 +210,12 @@ __global__ void k_ion_efix(Lay L, GridP g, Vec3P E) {
 // WindEFix (apps/wind.F90:489-565): edges i = ie-2 .. ie+1 blended toward the wind's -V x B, plus the
 // diffusive E of DiffuseOuter (:568-618) on the outermost edges
 struct Xyz3 { const double* x[3]; };
+// One thread per edge and direction (blockIdx.y); the J and K threads of the outermost edges each take the K edge's
+// weight for their diffusive term (E_I's is zero). One thread per edge with the three wind weights in turn took
+// 18.6 us at 96x96x128, now 13.1.
 __global__ void k_wind_efix(Lay L, Par p, GridP g, Xyz3 X, StateP n, Vec3P E, const Scal* sc) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int ni = 4, nj = L.Njp + 1, nk = L.Nkp + 1;
+    const int ni = 4, nj = L.Njp + 1, nk = L.Nkp + 1, d = blockIdx.y;
     if (t >= (long long)ni * nj * nk) return;
     const int i = L.ie() - 2 + (int)(t % ni);
     const long long q = t / ni;
@@ -215,66 +224,78 @@ __global__ void k_wind_efix(Lay L, Par p, GridP g, Xyz3 X, StateP n, Vec3P E, co
     double swE[3] = {-(m.wV[1] * m.wB[2] - m.wV[2] * m.wB[1]), -(m.wV[2] * m.wB[0] - m.wV[0] * m.wB[2]),
                      -(m.wV[0] * m.wB[1] - m.wV[1] * m.wB[0])};
     const long long c = L.at(i, j, k);
-    double wSW = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        const long long c2 = c + L.stride(d);
+    // the wind's weight at the centre of the edge of direction e, and that edge's vector
+    auto weight = [&](int e, double* de) {
+        const long long c2 = c + L.stride(e);
         double e1[3] = {X.x[0][c], X.x[1][c], X.x[2][c]}, e2[3] = {X.x[0][c2], X.x[1][c2], X.x[2][c2]};
         double ecc[3] = {0.5 * (e1[0] + e2[0]), 0.5 * (e1[1] + e2[1]), 0.5 * (e1[2] + e2[2])};
-        wSW = wgtWind(m, ecc);
-        if (wSW > TINY) {
-            if (i <= L.ie()) wSW = wSW / (1.0 + L.ie() + 1 - i);
-            double de[3] = {e2[0] - e1[0], e2[1] - e1[1], e2[2] - e1[2]};
-            E.v[d][c] = (1.0 - wSW) * E.v[d][c] + wSW * dot3v(swE, de);
+        for (int x = 0; x < 3; ++x) de[x] = e2[x] - e1[x];
+        double w = wgtWind(m, ecc);
+        if (w > TINY && i <= L.ie()) w = w / (1.0 + L.ie() + 1 - i);
+        return w;
+    };
+    double de[3], ed = E.v[d][c];
+    double wSW = weight(d, de);
+    if (wSW > TINY) ed = (1.0 - wSW) * ed + wSW * dot3v(swE, de);
+    if (i == L.ie() + 1) {   // DiffuseOuter with the weight of the last (K) edge
+        double dk[3];
+        if (d != 2) wSW = weight(2, dk);
+        if (d == 0) ed = ed + wSW * 0.0;
+        else {
+            const double vSW = dmin(norm2D(m.wV), p.Ca);
+            const long long cj = L.stride(1), ck = L.stride(2);
+            double db1, db2;
+            if (d == 2) {
+                db2 = n.mf[1][c] / dmax(g.face[1][c], TINY) - n.mf[1][c - 1] / dmax(g.face[1][c - 1], TINY);
+                db1 = n.mf[0][c] / g.face[0][c] - n.mf[0][c - cj] / g.face[0][c - cj];
+            } else {
+                db2 = n.mf[0][c] / g.face[0][c] - n.mf[0][c - ck] / g.face[0][c - ck];
+                db1 = n.mf[2][c] / g.face[2][c] - n.mf[2][c - 1] / g.face[2][c - 1];
+            }
+            double dl = sqrt(g.edge[1][c] * g.edge[2][c]);
+            double Vd = dmin(vSW, p.CFL * dl / sc->dt);
+            ed = ed + wSW * (Vd * (db2 - db1) * dl);
         }
     }
-    if (i == L.ie() + 1) {   // DiffuseOuter with the weight of the last (K) edge
-        const double vSW = dmin(norm2D(m.wV), p.Ca);
-        const long long cj = L.stride(1), ck = L.stride(2);
-        double bP = n.mf[1][c] / dmax(g.face[1][c], TINY), bM = n.mf[1][c - 1] / dmax(g.face[1][c - 1], TINY);
-        double db2 = bP - bM;
-        bP = n.mf[0][c] / g.face[0][c]; bM = n.mf[0][c - cj] / g.face[0][c - cj];
-        double db1 = bP - bM;
-        const double JdK = db2 - db1;
-        bP = n.mf[0][c] / g.face[0][c]; bM = n.mf[0][c - ck] / g.face[0][c - ck];
-        db2 = bP - bM;
-        bP = n.mf[2][c] / g.face[2][c]; bM = n.mf[2][c - 1] / g.face[2][c - 1];
-        db1 = bP - bM;
-        const double JdJ = db2 - db1;
-        double dl = sqrt(g.edge[1][c] * g.edge[2][c]);
-        double Vd = dmin(vSW, p.CFL * dl / sc->dt);
-        E.v[0][c] = E.v[0][c] + wSW * 0.0;
-        E.v[1][c] = E.v[1][c] + wSW * (Vd * JdJ * dl);
-        E.v[2][c] = E.v[2][c] + wSW * (Vd * JdK * dl);
-    }
+    E.v[d][c] = ed;
 }
-// WindEFix's touch-up next to the axis: the I edges of the axis rows take their k average, the K edges 0
-__global__ void k_wind_efix_ring(Lay L, Par p, Vec3P E) {
-    const int t = threadIdx.x;   // 4 shells x 2 sides
-    if (t >= 8) return;
+// the sum of a block's values over its threads (128), in the same order for every thread count in use
+__device__ __forceinline__ double blockSum(double v) {
+    __shared__ double ws[4];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return (ws[0] + ws[1]) + (ws[2] + ws[3]);
+}
+// WindEFix's touch-up next to the axis: the I edges of the axis rows take their k average, the K edges 0. A block
+// of 128 threads per shell (4) and side, threads along k: one thread each walked its ring twice, Nkp dependent
+// strided loads (38.4 us at Nkp = 128), now 3.4.
+__global__ void __launch_bounds__(128) k_wind_efix_ring(Lay L, Par p, Vec3P E) {
+    const int t = blockIdx.x;   // 4 shells x 2 sides
     const int nS = L.ie() - 2 + (t >> 1), side = t & 1;   // side 0: doE (je+1), 1: doS (js)
     if ((side == 0 && !p.ringDoE) || (side == 1 && !p.ringDoS)) return;
     const int j = side == 0 ? L.je() + 1 : L.js();
     double s = 0.0;
-    for (int k = L.ks(); k <= L.ke(); ++k) s = s + E.v[0][L.at(nS, j, k)];
-    const double avg = s / L.Nkp;
-    for (int k = 0; k < L.Nk; ++k) { E.v[0][L.at(nS, j, k)] = avg; E.v[2][L.at(nS, j, k)] = 0.0; }
+    for (int k = L.ks() + (int)threadIdx.x; k <= L.ke(); k += 128) s = s + E.v[0][L.at(nS, j, k)];
+    const double avg = blockSum(s) / L.Nkp;
+    for (int k = threadIdx.x; k < L.Nk; k += 128) { E.v[0][L.at(nS, j, k)] = avg; E.v[2][L.at(nS, j, k)] = 0.0; }
 }
 
 // ------------------------------------------------------------------ fluxes (HackFlux = IonFlux)
 // IonFlux (earthcmi.F90:282-331): the first shell's I fluxes at the two cells next to the axis replaced by
-// their average over k. One thread per side and variable (5 gas, 3 magnetic); doE before doS as there.
+// their average over k. A block of 128 threads, along k, per side and variable (5 gas, 3 magnetic); one thread
+// each took 26.8 us at Nkp = 128, now 3.6.
 template <typename O>
-__global__ void k_ion_flux(Lay L, Par p, FluxOut<O> FI) {
-    const int t = threadIdx.x;
-    if (t >= 16) return;
+__global__ void __launch_bounds__(128) k_ion_flux(Lay L, Par p, FluxOut<O> FI) {
+    const int t = blockIdx.x;
     const int side = t / 8, v = t % 8;   // side 0: je (doE), 1: js (doS)
     if ((side == 0 && !p.ringDoE) || (side == 1 && !p.ringDoS)) return;
     const int j = side == 0 ? L.je() : L.js();
     O* q = v < 5 ? FI.g[v] : FI.m[v - 5];
     double s = 0.0;
-    for (int k = L.ks(); k <= L.ke(); ++k) s = s + double(q[L.at(L.is(), j, k)]);
-    const O avg = O(s / L.Nkp);
-    for (int k = L.ks(); k <= L.ke(); ++k) q[L.at(L.is(), j, k)] = avg;
+    for (int k = L.ks() + (int)threadIdx.x; k <= L.ke(); k += 128) s = s + double(q[L.at(L.is(), j, k)]);
+    const O avg = O(blockSum(s) / L.Nkp);
+    for (int k = L.ks() + (int)threadIdx.x; k <= L.ke(); k += 128) q[L.at(L.is(), j, k)] = avg;
 }
 
 // ------------------------------------------------------------------ gravity
@@ -383,15 +404,17 @@ __global__ void k_nudge_ring(Lay L, Par p, StateP S) {
 }  // namespace
 
 // ------------------------------------------------------------------ launch helpers
-void launch_msph_bcs(Handle& h, const StateP& s, cudaStream_t st) {
+void launch_msph_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB) {
     const Lay& L = h.L;
     GridP g = h.gridP();
+    k_bc_ionwind<<<dim3(nblkM((long long)L.nG * (L.Nj + 1) * (L.Nk + 1), TB), 5), TB, 0, st>>>(L, h.p, g, s);
+    h.launches++;
+    if (!withB) return;   // a step rewrites every ghost B after its boundary conditions
     for (int side = 0; side < 2; ++side) {
         if (h.p.bc[side] != (side == 0 ? BC_ION : BC_WIND)) continue;
-        k_bc_ionwind<<<nblkM((long long)L.nG * (L.Nj + 1) * (L.Nk + 1), TB), TB, 0, st>>>(L, h.p, g, s, side);
         k_bc_ionwind_b<<<nblkM((long long)L.nG * L.Nj * L.Nk, TB), TB, 0, st>>>(L, h.p, g, s, side);
         k_bc_ionwind_bfix<<<nblkM((long long)L.nG * L.Nk, TB), TB, 0, st>>>(L, h.p, s, side);
-        h.launches += 3;
+        h.launches += 2;
     }
 }
 void launch_msph_efix(Handle& h, const StateP& nS, cudaStream_t st) {
@@ -401,9 +424,9 @@ void launch_msph_efix(Handle& h, const StateP& nS, cudaStream_t st) {
     if (h.p.bc[0] == BC_ION) { k_ion_efix<<<nblkM((long long)L.Nj * L.Nk, TB), TB, 0, st>>>(L, g, E); h.launches++; }
     if (h.p.bc[1] == BC_WIND) {
         Xyz3 X = {{h.xyz[0], h.xyz[1], h.xyz[2]}};
-        k_wind_efix<<<nblkM(4LL * (L.Njp + 1) * (L.Nkp + 1), TB), TB, 0, st>>>(L, h.p, g, X, nS, E, h.dScal);
+        k_wind_efix<<<dim3(nblkM(4LL * (L.Njp + 1) * (L.Nkp + 1), TB), 3), TB, 0, st>>>(L, h.p, g, X, nS, E, h.dScal);
         h.launches++;
-        if (h.p.doRing) { k_wind_efix_ring<<<1, 32, 0, st>>>(L, h.p, E); h.launches++; }
+        if (h.p.doRing) { k_wind_efix_ring<<<8, 128, 0, st>>>(L, h.p, E); h.launches++; }
     }
     launch_fix_e_lfm(h, h.E, st);   // FixEFieldLFM, EFix's last call
 }
@@ -413,8 +436,8 @@ void launch_ion_flux(Handle& h, cudaStream_t st) {
     FluxOut<double> F64;
     for (int v = 0; v < 5; ++v) { F32.g[v] = h.f32.gflx[0][v]; F64.g[v] = h.gflx[0][v]; }
     for (int x = 0; x < 3; ++x) { F32.m[x] = h.f32.mflx[0][x]; F64.m[x] = h.mflx[0][x]; }
-    if (h.prec == PREC_FP32FLUX) k_ion_flux<float><<<1, 32, 0, st>>>(h.L, h.p, F32);
-    else k_ion_flux<double><<<1, 32, 0, st>>>(h.L, h.p, F64);
+    if (h.prec == PREC_FP32FLUX) k_ion_flux<float><<<16, 128, 0, st>>>(h.L, h.p, F32);
+    else k_ion_flux<double><<<16, 128, 0, st>>>(h.L, h.p, F64);
     h.launches++;
 }
 void launch_apply_grav(Handle& h, const StateP& S, const StateP& O, cudaStream_t st) {
@@ -439,7 +462,7 @@ void launch_msph_perstep(Handle& h, const StateP& S, cudaStream_t st) {
 int msph_kernels_per_step(const Handle& h) {
     if (!h.p.msph.on) return 0;
     int n = 0;
-    for (int side = 0; side < 2; ++side) if (h.p.bc[side] == (side == 0 ? BC_ION : BC_WIND)) n += 3;
+    if (h.p.bc[0] == BC_ION || h.p.bc[1] == BC_WIND) n += 1;
     n += (h.p.bc[0] == BC_ION) + (h.p.bc[1] == BC_WIND) * (1 + (h.p.doRing ? 1 : 0)) + 1;   // EFix
     n += (h.p.bc[0] == BC_ION && h.p.doRing) ? 1 : 0;                                         // IonFlux
     n += h.p.msph.doGrav ? 1 : 0;

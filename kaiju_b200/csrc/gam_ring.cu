@@ -4,7 +4,7 @@
 //
 // A ring is the Np = Nkp cells around the axis at one radius (slice i) and one distance from the axis
 // (j = js+nR-1 or je-nR+1). One CTA owns one ring: the ring sits in shared memory, element-wise work is
-// spread over the threads, and the few sequential sums of the reference (Fourier coefficients, chunk
+// spread over the threads, each Fourier sum over a warp, and the other sequential sums of the reference (chunk
 // sums, the intra-chunk running flux) run on one thread each, in the reference's order.
 #include <cstdio>
 #include "gam_common.cuh"
@@ -106,22 +106,50 @@ __global__ void k_ring_flux_kavg(Lay L, FluxOut<O> FK) {
 }
 
 // ------------------------------------------------------------------ PoleE (ringav.F90:376-411) + FixEFieldLFM
-// On the axis edges E_K = 0 and E_I is its ring mean (every k of the array)
-__global__ void k_pole_e(Lay L, Par p, Vec3P E) {
-    int nS = L.is() + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (nS > L.ie() + 1) return;
-    for (int side = 0; side < 2; ++side) {
-        if (side == 0 && !p.ringDoS) continue;
-        if (side == 1 && !p.ringDoE) continue;
-        int j = side == 0 ? L.js() : L.je() + 1;
-        double s = 0.0;
-        for (int k = L.ks(); k <= L.ke(); ++k) s = s + E.v[0][L.at(nS, j, k)];
-        double avg = s / L.Nkp;
-        for (int k = 0; k < L.Nk; ++k) {
-            long long c = L.at(nS, j, k);
-            E.v[2][c] = 0.0;
-            E.v[0][c] = avg;
+// Sum over the active k of a k-plane stack's (i, j) column: a block of 32 columns (threadIdx.x, along i) by 8 rows
+// of threads that share each column's k range; every thread of a column returns the sum.
+__device__ __forceinline__ double axisSum(const double* q, const Lay& L, int i, int j, bool in) {
+    __shared__ double part[8][33];
+    double s = 0.0;
+    if (in)
+        for (int k = L.ks() + (int)threadIdx.y; k <= L.ke(); k += 8) s = s + q[L.at(i, j, k)];
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    s = 0.0;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) s = s + part[y][threadIdx.x];
+    return s;
+}
+// On the axis edges E_K = 0 and E_I is its ring mean (every k of the array): blockIdx.y < 2 (side), 32 i by 8 k
+// threads. FixEFieldLFM (gamdebug.F90:149-175; E_I and E_J at ks and ke+1 take their mean) in the same launch,
+// blockIdx.y >= 2, one row of threads per j: it leaves the axis rows' E_I alone, whose planes PoleE makes equal.
+// One thread per i that walked its ring took 30.8 us at 96x96x128 and Nkp = 128 and 3.4 us for the second launch,
+// now 10.9.
+__global__ void __launch_bounds__(256) k_pole_e(Lay L, Par p, Vec3P E) {
+    const int i = L.is() + (int)(blockIdx.x * 32 + threadIdx.x);
+    const bool in = i <= L.ie() + 1;
+    if (blockIdx.y >= 2) {
+        const int j = L.js() + (int)((blockIdx.y - 2) * 8 + threadIdx.y);
+        if (!in || j > L.je() + 1) return;
+        const bool axis = (p.ringDoS && j == L.js()) || (p.ringDoE && j == L.je() + 1);
+        const long long c0 = L.at(i, j, L.ks()), c1 = L.at(i, j, L.ke() + 1);
+        const double Ej = 0.5 * (E.v[1][c0] + E.v[1][c1]);
+        if (!axis) {
+            const double Ei = 0.5 * (E.v[0][c0] + E.v[0][c1]);
+            E.v[0][c0] = Ei; E.v[0][c1] = Ei;
         }
+        E.v[1][c0] = Ej; E.v[1][c1] = Ej;
+        return;
+    }
+    const int side = blockIdx.y;
+    if ((side == 0 && !p.ringDoS) || (side == 1 && !p.ringDoE)) return;
+    const int j = side == 0 ? L.js() : L.je() + 1;
+    const double avg = axisSum(E.v[0], L, i, j, in) / L.Nkp;
+    if (!in) return;
+    for (int k = threadIdx.y; k < L.Nk; k += 8) {
+        long long c = L.at(i, j, k);
+        E.v[2][c] = 0.0;
+        E.v[0][c] = avg;
     }
 }
 // FixEFieldLFM (gamdebug.F90:149-175): E_I and E_J at ks and ke+1 take their mean
@@ -201,18 +229,17 @@ __device__ void ringReconstruct(double* rW, int Np, int Nc, int meth) {
 }
 // CleanRing / DirtyRing (ringav.F90:416-458) with the trigonometric table of the ring in shared memory
 // (cosT[m*Np+n] = cos(m*phi_n), sinT likewise); cFT in shared memory
+// One warp per Fourier sum (RTPB threads, 2 (numFT + 1) sums): one thread that took all of them in turn was most
+// of the 65 us that each pole's k_ring_smooth_e took at 96x96x128; both poles in one launch now 30.9.
 __device__ void ringClean(double* Q, const double* cosT, const double* sinT, double* cFT, int Np, int numFT) {
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double aScl = (double)(2.0f / (float)Np);
-        for (int m = 0; m <= NFTMAX; ++m) { cFT[2 * m] = 0.0; cFT[2 * m + 1] = 0.0; }
-        for (int n = 0; n < Np; ++n)
-            for (int m = 0; m <= numFT; ++m) {
-                cFT[2 * m] = cFT[2 * m] + Q[n] * cosT[m * Np + n];
-                cFT[2 * m + 1] = cFT[2 * m + 1] + Q[n] * sinT[m * Np + n];
-            }
-        cFT[0] = 0.5 * aScl * cFT[0]; cFT[1] = 0.5 * aScl * cFT[1];
-        for (int m = 1; m <= numFT; ++m) { cFT[2 * m] = 1.0 * aScl * cFT[2 * m]; cFT[2 * m + 1] = 1.0 * aScl * cFT[2 * m + 1]; }
+    const double aScl = (double)(2.0f / (float)Np);
+    for (int q = threadIdx.x >> 5; q < 2 * (numFT + 1); q += RTPB / 32) {
+        const double* tab = ((q & 1) ? sinT : cosT) + (q >> 1) * Np;
+        double s = 0.0;
+        for (int n = threadIdx.x & 31; n < Np; n += 32) s = s + Q[n] * tab[n];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == 0) cFT[q] = (q < 2 ? 0.5 : 1.0) * aScl * s;
     }
     __syncthreads();
     for (int n = threadIdx.x; n < Np; n += blockDim.x) {
@@ -233,8 +260,9 @@ __device__ void ringDirty(double* Q, const double* cosT, const double* sinT, con
 }
 
 // ------------------------------------------------------------------ CalcSmoothE (ringav.F90:203-336), LFM axis
-// grid: (nS = is..ie+1) x (nR = 1..NumR); pole 0 = SPOLE (+x), 1 = EPOLE (-x)
-__global__ void __launch_bounds__(RTPB) k_ring_smooth_e(Lay L, RingDev R, StateP s, Vec3P SE, int pole) {
+// grid: (nS = is..ie+1) x (nR = 1..NumR) x poles; pole 0 = SPOLE (+x), 1 = EPOLE (-x)
+__global__ void __launch_bounds__(RTPB) k_ring_smooth_e(Lay L, RingDev R, StateP s, Vec3P SE, int pole0) {
+    const int pole = pole0 + blockIdx.z;
     extern __shared__ __align__(16) double rsm[];
     const int Np = R.Np;
     double* cosT = rsm;                       // (NFTMAX+1)*Np
@@ -249,7 +277,7 @@ __global__ void __launch_bounds__(RTPB) k_ring_smooth_e(Lay L, RingDev R, StateP
     const double dp = 2.0 * PI / Np;
     for (int n = threadIdx.x; n < Np; n += blockDim.x) {
         double phi = dp * (n + 1) - 0.5 * dp;
-        for (int m = 0; m <= NFTMAX; ++m) { cosT[m * Np + n] = cos(1.0 * m * phi); sinT[m * Np + n] = sin(1.0 * m * phi); }
+        for (int m = 0; m <= R.NFTMAG; ++m) { cosT[m * Np + n] = cos(1.0 * m * phi); sinT[m * Np + n] = sin(1.0 * m * phi); }
         int k = L.ks() + n;
         if (pole == 0) {   // PullRingI (ringutils.F90:753-787)
             bFlx[n] = s.mf[0][L.at(nS, L.js() + nR - 1, k)];
@@ -318,26 +346,24 @@ __global__ void k_e2flux_inplace(Lay L, Vec3P E, StateP s) {
 }
 
 // ------------------------------------------------------------------ CleanLoops (ringav.F90:339-373), LFM axis
-__global__ void k_clean_loops(Lay L, Par p, StateP s, double tScl) {
-    int nS = L.is() + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (nS > L.ie() + 1) return;
-    for (int side = 0; side < 2; ++side) {
-        if (side == 0 && !p.ringDoS) continue;
-        if (side == 1 && !p.ringDoE) continue;
-        int j = side == 0 ? L.js() : L.je();
-        double sum = 0.0;
-        for (int k = L.ks(); k <= L.ke(); ++k) sum = sum + s.mf[2][L.at(nS, j, k)];
-        double avgFlx = sum / L.Nkp;
-        for (int k = L.ks(); k <= L.ke() + 1; ++k) {
-            long long c = L.at(nS, j, k);
-            s.mf[2][c] = s.mf[2][c] - tScl * avgFlx;
-        }
+// blockIdx.y = side, 32 i by 8 k threads; one thread per i took 40.2 us at 96x96x128, now 8.8
+__global__ void __launch_bounds__(256) k_clean_loops(Lay L, Par p, StateP s, double tScl) {
+    const int i = L.is() + (int)(blockIdx.x * 32 + threadIdx.x), side = blockIdx.y;
+    const bool in = i <= L.ie() + 1;
+    if ((side == 0 && !p.ringDoS) || (side == 1 && !p.ringDoE)) return;
+    const int j = side == 0 ? L.js() : L.je();
+    const double avgFlx = axisSum(s.mf[2], L, i, j, in) / L.Nkp;
+    if (!in) return;
+    for (int k = L.ks() + (int)threadIdx.y; k <= L.ke() + 1; k += 8) {
+        long long c = L.at(i, j, k);
+        s.mf[2][c] = s.mf[2][c] - tScl * avgFlx;
     }
 }
 
 // ------------------------------------------------------------------ SmoothGas (ringav.F90:82-200), single fluid
-// grid: (nS = is..ie) x (nR = 1..NumR)
-__global__ void __launch_bounds__(RTPB) k_ring_smooth_gas(Lay L, Par p, RingDev R, StateP s, int pole) {
+// grid: (nS = is..ie) x (nR = 1..NumR) x poles
+__global__ void __launch_bounds__(RTPB) k_ring_smooth_gas(Lay L, Par p, RingDev R, StateP s, int pole0) {
+    const int pole = pole0 + blockIdx.z;
     extern __shared__ __align__(16) double rsm[];
     const int Np = R.Np;
     double* rW = rsm;            // 5*Np
@@ -471,9 +497,8 @@ void launch_ring_flux(Handle& h, cudaStream_t st) {
 void launch_pole_e(Handle& h, double* const* E, cudaStream_t st) {
     const Lay& L = h.L;
     Vec3P e = {{E[0], E[1], E[2]}};
-    k_pole_e<<<nblk1(L.Nip + 1, 64), 64, 0, st>>>(L, h.p, e);
-    k_fix_e_lfm<<<nblk1((long long)(L.Nip + 1) * (L.Njp + 1), 256), 256, 0, st>>>(L, e);
-    h.launches += 2;
+    k_pole_e<<<dim3(nblk1(L.Nip + 1, 32), 2 + nblk1(L.Njp + 1, 8)), dim3(32, 8), 0, st>>>(L, h.p, e);
+    h.launches++;
 }
 void launch_fix_e_lfm(Handle& h, double* const* E, cudaStream_t st) {
     const Lay& L = h.L;
@@ -488,33 +513,42 @@ void launch_ring_average(Handle& h, const StateP& s, cudaStream_t st) {
     Vec3P SE = {{h.SmoothE[0], h.SmoothE[1], h.SmoothE[2]}};
     cudaMemsetAsync(h.SmoothE[0], 0, sizeof(double) * L.E * 3, st);   // InitRAVec: contiguous planes
     h.launches++;
-    dim3 ge((unsigned)(L.Nip + 1), (unsigned)R.NumR);
-    if (p.ringDoS) { k_ring_smooth_e<<<ge, RTPB, smoothESmem(R.Np), st>>>(L, R, s, SE, 0); h.launches++; }
-    if (p.ringDoE) { k_ring_smooth_e<<<ge, RTPB, smoothESmem(R.Np), st>>>(L, R, s, SE, 1); h.launches++; }
+    // the poles' rings are different rows as long as they do not meet: one launch for both, else one after the other
+    const bool both = p.ringDoS && p.ringDoE && 2 * R.NumR < L.Njp;
+    for (int pole = 0; pole < 2; ++pole) {
+        if (!(pole == 0 ? p.ringDoS : p.ringDoE) || (both && pole == 1)) continue;
+        const dim3 ge((unsigned)(L.Nip + 1), (unsigned)R.NumR, both ? 2 : 1);
+        k_ring_smooth_e<<<ge, RTPB, smoothESmem(R.Np), st>>>(L, R, s, SE, pole);
+        h.launches++;
+    }
     launch_pole_e(h, h.SmoothE, st);
     long long nf = (long long)(L.Nip + 1) * (L.Njp + 1) * (L.Nkp + 1);
     k_e2flux_inplace<<<nblk1(nf, 256), 256, 0, st>>>(L, SE, s);
     h.launches++;
     if (h.ring.doCleanLoop) {
         double tScl = h.ring.doFastLoop ? 1.0 : 1.0 / L.Nkp;
-        k_clean_loops<<<nblk1(L.Nip + 1, 64), 64, 0, st>>>(L, p, s, tScl);
+        k_clean_loops<<<dim3(nblk1(L.Nip + 1, 32), 2), dim3(32, 8), 0, st>>>(L, p, s, tScl);
         h.launches++;
     }
     launch_bflux2fld(h, s, st);   // includes the ring fix
-    dim3 gg((unsigned)L.Nip, (unsigned)R.NumR);
-    if (p.ringDoS) { k_ring_smooth_gas<<<gg, RTPB, smoothGasSmem(R.Np), st>>>(L, p, R, s, 0); h.launches++; }
-    if (p.ringDoE) { k_ring_smooth_gas<<<gg, RTPB, smoothGasSmem(R.Np), st>>>(L, p, R, s, 1); h.launches++; }
+    for (int pole = 0; pole < 2; ++pole) {
+        if (!(pole == 0 ? p.ringDoS : p.ringDoE) || (both && pole == 1)) continue;
+        const dim3 gg((unsigned)L.Nip, (unsigned)R.NumR, both ? 2 : 1);
+        k_ring_smooth_gas<<<gg, RTPB, smoothGasSmem(R.Np), st>>>(L, p, R, s, pole);
+        h.launches++;
+    }
 }
 
 int ring_kernels_per_step(const Handle& h) {
     if (!h.p.doRing) return 0;
     const Par& p = h.p;
-    int sides = (p.ringDoS ? 1 : 0) + (p.ringDoE ? 1 : 0);
+    const bool both = p.ringDoS && p.ringDoE && 2 * h.ring.NumR < h.L.Njp;
+    int sides = both ? 1 : (p.ringDoS ? 1 : 0) + (p.ringDoE ? 1 : 0);
     int n = 0;
     n += 1 + (p.predFixLFM ? 1 : 0);                    // predictor: ring fix (+ PredFix)
     n += 1 + (p.doMHD ? 1 : 0);                         // RingFlux
-    if (p.doMHD) n += 2;                                // PoleE on the step E
-    n += 1 + sides + 2 + 1 + (h.ring.doCleanLoop ? 1 : 0) + 2 + sides;   // RingAverage
+    if (p.doMHD) n += 1;                                // PoleE on the step E
+    n += 1 + sides + 1 + 1 + (h.ring.doCleanLoop ? 1 : 0) + 2 + sides;   // RingAverage
     n += 1;                                             // ring fix after the final bFlux2Fld
     return n;
 }

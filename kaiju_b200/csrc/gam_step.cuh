@@ -108,7 +108,8 @@ void launch_dt_finalize(Handle& h, int mode, cudaStream_t st);
 enum { PH_PREDICT = 0, PH_EFIELD, PH_FLUXES, PH_DELTAS, PH_UPDATE, PH_DT, PH_BCS, NPHASE };
 // Kernels used outside the step
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st);
-void launch_bcs(Handle& h, const StateP& s, cudaStream_t st);
+// withB: ghost B copied with the gas (set-up); a step leaves it to the bFlux2Fld of the ghost cells that follows
+void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB = true);
 void launch_calcdt(Handle& h, const StateP& s, int mode, cudaStream_t st);   // mode 0: in-step, 1: initial (no time advance)
 double launch_divb(Handle& h, double* scratchDev, cudaStream_t st);
 int kernels_per_step(const Handle& h);
@@ -137,7 +138,7 @@ void launch_ring_flux(Handle& h, cudaStream_t st);                              
 void launch_pole_e(Handle& h, double* const* E, cudaStream_t st);               // PoleE + FixEFieldLFM
 void launch_fix_e_lfm(Handle& h, double* const* E, cudaStream_t st);            // FixEFieldLFM alone
 // the magnetosphere problem (gam_msph.cu): its I boundaries, EFix, IonFlux, gravity and PerStep hooks
-void launch_msph_bcs(Handle& h, const StateP& s, cudaStream_t st);
+void launch_msph_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB);
 void launch_msph_efix(Handle& h, const StateP& nS, cudaStream_t st);
 void launch_ion_flux(Handle& h, cudaStream_t st);
 void launch_apply_grav(Handle& h, const StateP& S, const StateP& O, cudaStream_t st);
