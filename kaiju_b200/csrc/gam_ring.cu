@@ -196,41 +196,38 @@ __device__ void ringLR(int meth, double fm2, double fm1, double f, double fp1, d
     }
     vp = f + ap; vm = f + am;
 }
-// Chunk averages (each chunk's sum by one thread, in order)
-__device__ void ringChunkAvg(const double* in, double* out, int Np, int Nc) {
-    int dC = Np / Nc;
-    for (int n = threadIdx.x; n < Nc; n += blockDim.x) {
+// Chunk averages of nv rings (pitch Np), each chunk's sum by one thread, in order; avg[v * Np + n] is chunk n's
+__device__ void ringChunkAvg(const double* in, double* avg, int nv, int Np, int Nc) {
+    const int dC = Np / Nc;
+    for (int q = threadIdx.x; q < nv * Nc; q += blockDim.x) {
+        const int v = q / Nc, n = q - v * Nc;
         double s = 0.0;
-        for (int m = 0; m < dC; ++m) s = s + in[n * dC + m];
-        double a = s / dC;
-        for (int m = 0; m < dC; ++m) out[n * dC + m] = a;
+        for (int m = 0; m < dC; ++m) s = s + in[v * Np + n * dC + m];
+        avg[v * Np + n] = s / dC;
     }
-}
-// ReconstructRing (ringrecon.F90:34-98) of a chunk-averaged ring in place; every element evaluates the
-// parabola of its chunk from the chunk values (periodic, two ghost chunks)
-__device__ void ringReconstruct(double* rW, int Np, int Nc, int meth) {
-    int dJ = Np / Nc;
     __syncthreads();
-    double vals[8];   // Np / blockDim <= 512 / 128
-    int cnt = 0;
-    for (int e = threadIdx.x; e < Np; e += blockDim.x) {
-        int n = e / dJ, m = e % dJ + 1;
-        auto ch = [&](int q) { q = ((q % Nc) + Nc) % Nc; return rW[q * dJ]; };
+}
+// ReconstructRing (ringrecon.F90:34-98) of nv chunk-averaged rings: every element evaluates the parabola of its
+// chunk from the chunk values (periodic, two ghost chunks). The averages lie beside the result, so all rings go
+// through one pass without a barrier between them (the five gas rings one after the other, in place: k_ring_smooth_gas
+// 45.8 us for both poles at 96x96x128, now 36.5).
+__device__ void ringReconstruct(const double* avg, double* out, int nv, int Np, int Nc, int meth) {
+    const int dJ = Np / Nc;
+    for (int t = threadIdx.x; t < nv * Np; t += blockDim.x) {
+        const int v = t / Np, e = t - v * Np, n = e / dJ, m = e - n * dJ + 1;
+        auto ch = [&](int q) { return avg[v * Np + ((q % Nc) + Nc) % Nc]; };
         double f = ch(n), fL, fR;
         ringLR(meth, ch(n - 2), ch(n - 1), f, ch(n + 1), ch(n + 2), fL, fR);
         double a = 3 * (fL + fR - 2 * f), b = 2 * (3 * f - fR - 2 * fL), c = fL;
-        vals[cnt++] = (a / 3.0) * (double)(3 * m * m - 3 * m + 1) / (double)(dJ * dJ) +
-                      0.5 * b * (double)(2 * m - 1) / (double)dJ + c;
+        out[t] = (a / 3.0) * (double)(3 * m * m - 3 * m + 1) / (double)(dJ * dJ) +
+                 0.5 * b * (double)(2 * m - 1) / (double)dJ + c;
     }
-    __syncthreads();
-    cnt = 0;
-    for (int e = threadIdx.x; e < Np; e += blockDim.x) rW[e] = vals[cnt++];
     __syncthreads();
 }
 // CleanRing / DirtyRing (ringav.F90:416-458) with the trigonometric table of the ring in shared memory
 // (cosT[m*Np+n] = cos(m*phi_n), sinT likewise); cFT in shared memory
 // One warp per Fourier sum (RTPB threads, 2 (numFT + 1) sums): one thread that took all of them in turn was most
-// of the 65 us that each pole's k_ring_smooth_e took at 96x96x128; both poles in one launch now 30.9.
+// of the 65 us that each pole's k_ring_smooth_e took at 96x96x128; both poles in one launch now 30.8.
 __device__ void ringClean(double* Q, const double* cosT, const double* sinT, double* cFT, int Np, int numFT) {
     __syncthreads();
     const double aScl = (double)(2.0f / (float)Np);
@@ -271,7 +268,8 @@ __global__ void __launch_bounds__(RTPB) k_ring_smooth_e(Lay L, RingDev R, StateP
     double* rFlx = bFlx + 3 * Np;             // Np
     double* raFlx = rFlx + Np;                // Np
     double* dEr = raFlx + Np;                 // 2*Np (I, J)
-    double* cFT = dEr + 2 * Np;               // 2*(NFTMAX+1)
+    double* avg = dEr + 2 * Np;               // Np
+    double* cFT = avg + Np;                   // 2*(NFTMAX+1)
     const int nS = L.is() + blockIdx.x, nR = 1 + blockIdx.y;
     const int NumCh = R.Nch[nR - 1], dC = Np / NumCh;
     const double dp = 2.0 * PI / Np;
@@ -295,8 +293,8 @@ __global__ void __launch_bounds__(RTPB) k_ring_smooth_e(Lay L, RingDev R, StateP
         __syncthreads();
         for (int n = threadIdx.x; n < Np; n += blockDim.x) rFlx[n] = bFlx[fD * Np + n];
         ringClean(rFlx, cosT, sinT, cFT, Np, R.NFTMAG);
-        ringChunkAvg(rFlx, raFlx, Np, NumCh);
-        ringReconstruct(raFlx, Np, NumCh, R.recon);
+        ringChunkAvg(rFlx, avg, 1, Np, NumCh);
+        ringReconstruct(avg, raFlx, 1, Np, NumCh, R.recon);
         ringDirty(raFlx, cosT, sinT, cFT, Np, R.NFTMAG);
         // running flux change within each chunk -> ring E (one thread per chunk, in order)
         for (int n = threadIdx.x; n < NumCh; n += blockDim.x) {
@@ -366,8 +364,8 @@ __global__ void __launch_bounds__(RTPB) k_ring_smooth_gas(Lay L, Par p, RingDev 
     const int pole = pole0 + blockIdx.z;
     extern __shared__ __align__(16) double rsm[];
     const int Np = R.Np;
-    double* rW = rsm;            // 5*Np
-    double* raW = rW + 5 * Np;   // 5*Np
+    double* rW = rsm;            // 5*Np: the ring, then its smoothed values
+    double* avg = rW + 5 * Np;   // 5*Np: chunk averages
     const int nS = L.is() + blockIdx.x, nR = 1 + blockIdx.y;
     const int NumCh = R.Nch[nR - 1];
     const int jR = pole == 0 ? L.js() + nR - 1 : L.je() - nR + 1;
@@ -382,12 +380,12 @@ __global__ void __launch_bounds__(RTPB) k_ring_smooth_gas(Lay L, Par p, RingDev 
         rW[4 * Np + n] = R.doMassRA ? p.gamma * P : P / gm1;
     }
     __syncthreads();
-    for (int v = 0; v < 5; ++v) ringChunkAvg(rW + v * Np, raW + v * Np, Np, NumCh);
-    for (int v = 0; v < 5; ++v) ringReconstruct(raW + v * Np, Np, NumCh, R.recon);
+    ringChunkAvg(rW, avg, 5, Np, NumCh);
+    ringReconstruct(avg, rW, 5, Np, NumCh, R.recon);
     for (int n = threadIdx.x; n < Np; n += blockDim.x) {   // Ring2Gas (ringutils.F90:829-856) + PushRingCC
-        double D = dmax(raW[n], p.dFloor);
-        double Mx = raW[Np + n], My = raW[2 * Np + n], Mz = raW[3 * Np + n];
-        double P = R.doMassRA ? (raW[4 * Np + n] / D) * D / p.gamma : gm1 * raW[4 * Np + n];
+        double D = dmax(rW[n], p.dFloor);
+        double Mx = rW[Np + n], My = rW[2 * Np + n], Mz = rW[3 * Np + n];
+        double P = R.doMassRA ? (rW[4 * Np + n] / D) * D / p.gamma : gm1 * rW[4 * Np + n];
         P = dmax(P, p.pFloor);
         double KinE = 0.5 * (Mx * Mx + My * My + Mz * Mz) / D;
         long long c = L.at(nS, jR, L.ks() + n);
@@ -453,7 +451,7 @@ void launch_ring_grid_fix(Handle& h, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ launchers
-static size_t smoothESmem(int Np) { return sizeof(double) * ((size_t)2 * (NFTMAX + 1) * Np + 7 * (size_t)Np + 2 * (NFTMAX + 1)); }
+static size_t smoothESmem(int Np) { return sizeof(double) * ((size_t)2 * (NFTMAX + 1) * Np + 8 * (size_t)Np + 2 * (NFTMAX + 1)); }
 static size_t smoothGasSmem(int Np) { return sizeof(double) * 10 * (size_t)Np; }
 
 void ring_kernels_init() {
