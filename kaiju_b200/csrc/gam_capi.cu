@@ -199,7 +199,7 @@ int alloc_handle(gam_gpu* G, const gam_model_c* m) {
     ring_kernels_init();
     CK(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     h.ownStream = true;
-    const size_t planes = 11 * 3 + 10 + 14 + 9 + 24 + 91 + 6;   // + the I and J edges' face velocities
+    const size_t planes = 11 * 3 + 10 + 11 + 9 + 24 + 91 + 6;   // + the I and J edges' face velocities
     h.poolPlanes = planes;
     CK(cudaMalloc(&h.pool, sizeof(double) * L.E * planes));
     CK(cudaMemsetAsync(h.pool, 0, sizeof(double) * L.E * planes, h.stream));
@@ -218,7 +218,6 @@ int alloc_handle(gam_gpu* G, const gam_model_c* m) {
     for (int x = 0; x < 3; ++x) h.E[x] = take();   // contiguous: memset as one range
     for (int x = 0; x < 3; ++x) h.Vf[x] = take();
     for (int e = 0; e < 2; ++e) for (int x = 0; x < 3; ++x) h.VfE[e][x] = take();
-    for (int x = 0; x < 3; ++x) h.VdV[x] = take();
     for (int x = 0; x < 3; ++x) h.hbA[x] = take();
     for (int x = 0; x < 3; ++x) h.nbA[x] = take();
     for (int v = 0; v < 5; ++v) h.dGasH[v] = take();
@@ -268,6 +267,7 @@ int alloc_handle(gam_gpu* G, const gam_model_c* m) {
     std::memset(h.hScal, 0, sizeof(Scal));
     h.hScal->t = m->t; h.hScal->dt = m->dt; h.hScal->dt0 = m->dt0; h.hScal->ts = m->ts;
     h.hScal->dtMinBits = 0x7FF0000000000000ull;
+    h.hScal->bGiven = B_GIVEN_STEPS;
     CK(cudaMemcpyAsync(h.dScal, h.hScal, sizeof(Scal), cudaMemcpyHostToDevice, h.stream));
     CK(cudaStreamSynchronize(h.stream));
     return GAM_OK;
@@ -491,6 +491,8 @@ int gam_gpu_sync_to_device(gam_gpu_t* G, unsigned what, const double* gas, const
         else launch_bflux2fld(h, o, h.stream);
     }
     if (rc) return rc;
+    // a state whose Bxyz was made from its fluxes just now needs no check
+    launch_b_check(h, !((what & GAM_SYNC_STATE) && !bxyz), !((what & GAM_SYNC_OSTATE) && !obxyz), h.stream);
     // State%time / oState%time travel with the arrays; the other scalars stay as they are on the device
     rc = download_scalars(G);
     if (rc) return rc;
@@ -722,7 +724,10 @@ int gam_gpu_fetch(gam_gpu_t* G, const char* name, double* out, long long n) {
     else if (s == "ogas") put(oS.gas, 5);
     else if (s == "omagflux") { put(oS.mf, 3); e = fe; }
     else if (s == "obxyz") put(oS.b, 3);
-    else if (s == "hgas") put(h.H.gas, 5);
+    else if (s == "hgas") {
+        if (h.prec == PREC_FP64 && !h.p.doBoris) launch_half_con(h, h.stream);
+        put(h.H.gas, 5);
+    }
     else if (s == "hmagflux") { put(h.H.mf, 3); e = fe; }
     else if (s == "hbxyz") put(h.H.b, 3);
     else if (s == "efld") put(h.E, 3);

@@ -1023,9 +1023,9 @@ int gam_gpu_restrict(gam_gpu_t* fine, gam_gpu_t* coarse, unsigned what) {
                                                                                                         hf.S[hf.cur], dst);
     launch_bcs(hc, dst, hc.stream);
     launch_bflux2fld(hc, dst, hc.stream);
+    launch_b_check(hc, true, true, hc.stream);
     hc.launches += 2;
-    CKC(cudaStreamSynchronize(hc.stream));
-    return GAM_OK;
+    return capi_download_scalars(coarse);   // with Scal::bGiven, and waits for the stream
 }
 
 int gam_closure_residual_rms(gam_closure_t* C, int slot, double* rms) {

@@ -68,6 +68,7 @@ struct Par {
     unsigned int stageWait;
     MsphPar msph;
 };
+constexpr int B_GIVEN_STEPS = 2;   // Scal::bGiven after a state came from outside: it is n, then n-1, in the next two
 constexpr unsigned int STAGE_WAIT = 1u << 20;
 constexpr unsigned int STAGE_DRAIN = 1u << 28;
 
@@ -81,7 +82,9 @@ struct Scal {
     int status;                       // status bits of the last CalcDT (1 disaster, 2 bad, 4 NaN, 8 wait gave up)
     int sticky;                       // OR of status over steps since the last reset
     unsigned int lastNan;             // nanCount of the last CalcDT
-    int pad;
+    // steps left whose predictor takes the half-state cell field from the face fluxes itself: the Bxyz of State n or
+    // oState came from outside the step (set-up, the host, a restriction) and need not be bFlux2Fld of its fluxes
+    int bGiven;
     // tiled runs: {dtMinBits, ~nanCount} of this tile, reduced with MIN across the tiles (so the second
     // word carries the largest NaN count) before the dt is finalized
     unsigned long long red[2];

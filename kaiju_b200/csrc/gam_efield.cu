@@ -1,9 +1,9 @@
 // Constrained-transport electric field (fields.F90:70-232) with shared-memory staging.
 //
 // For each edge direction eD with transverse pair (dT1, dT2) = (J,K), (K,I), (I,J):
-//  1. Vf on the dT1 faces, the volume-weighted Central8 of the cell values vol*rho*v/max(rho,dFloor)
-//     (precomputed once per cell by the predictor) over max(Central8(vol),TINY) -- one pass,
-//     k_mom2face3, for all three directions.
+//  1. Vf on the dT1 faces, the volume-weighted Central8 of the half-state velocities (the reference's
+//     vol*rho*v/max(rho,dFloor) summands) over max(Central8(vol),TINY) -- one pass, k_mom2face3, for all
+//     three directions.
 //  2. k_edge_tile: a CTA of 256 threads owns a 32 x TJ x TK tile of eD edges. It stages (TMA tensor copies,
 //     or cp.async) the stencil footprints -- along dT2: Vf, the dT1 face areas and the dT1 face field
 //     (flux/area, half state for the reconstruction, n state for the limiter); along dT1: the dT2 face
@@ -15,16 +15,17 @@ namespace gam {
 
 // ------------------------------------------------------------------ Mom2Face (fields.F90:235-285)
 struct Vec3F { float* v[3]; };
-// Vf at one face (explicit fused multiply-adds): the Central8 sums along dT1 of the summands
-// vol*rho*v/max(rho,dFloor) over the Central8 sum of the volumes (clamped at TINY). A is the accumulation type: double on the FP64 path, float on the
-// FP32-flux path, whose summands and volumes are float copies and whose Vf is stored as float.
+// Vf at one face (explicit fused multiply-adds): the Central8 sums along dT1 of volume * velocity over that of the
+// volumes (clamped at TINY), each weight applied to its volume once for the four sums. A is the accumulation type:
+// double on the FP64 path, float on the FP32-flux path, whose velocities and volumes are float copies and whose Vf
+// is stored as float.
 template <typename A>
 __device__ __forceinline__ void mom2face_sum(const A* wV, const A* w0, const A* w1, const A* w2, A& f0, A& f1, A& f2) {
     A sV = A(0), s0 = A(0), s1 = A(0), s2 = A(0);
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-        A w = A(wC8(n));
-        sV = fma(w, wV[n], sV);
+        A w = A(wC8(n)) * wV[n];
+        sV = sV + w;
         s0 = fma(w, w0[n], s0);
         s1 = fma(w, w1[n], s1);
         s2 = fma(w, w2[n], s2);
@@ -76,7 +77,6 @@ void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st) {
     const Lay& L = h.L;
     // E = 0 (fields.F90:88) needs no pass per step: the edge kernels rewrite the same edges every step, and
     // every edge outside them stays zero from the pool's zeroing (initialisation clears its scratch use)
-    Vec3P VdV = {{h.VdV[0], h.VdV[1], h.VdV[2]}};
     GridP g = h.gridP();
     EdgeSrc<double> in64;
     EdgeSrc<float> in32;
@@ -89,7 +89,7 @@ void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st) {
             for (int c = 0; c < 4; ++c) in32.Teb[d][c] = f.Teb[d][c];
             for (int c = 0; c < 2; ++c) in32.edgB0[d][c] = f.edgB0[d][c];
         }
-        in32.rho = f.rho;
+        in32.rho = f.Wh[0];
     } else {
         for (int x = 0; x < 3; ++x) in64.Vf[x] = h.Vf[x];
         for (int d = 0; d < 3; ++d) {
@@ -98,7 +98,7 @@ void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st) {
             for (int c = 0; c < 4; ++c) in64.Teb[d][c] = h.Teb[d][c];
             for (int c = 0; c < 2; ++c) in64.edgB0[d][c] = h.edgB0[d][c];
         }
-        in64.rho = h.H.gas[0];
+        in64.rho = h.Wh[0];
     }
     int is = L.is(), ie = L.ie(), js = L.js(), je = L.je(), ks = L.ks(), ke = L.ke();
     bool f32 = h.prec == PREC_FP32FLUX;
@@ -111,14 +111,14 @@ void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st) {
     if (f32) {
         Vf9<float> o;
         for (int x = 0; x < 3; ++x) { o.v[0][x] = h.f32.VfE[0][x]; o.v[1][x] = h.f32.VfE[1][x]; o.v[2][x] = h.f32.Vf[x]; }
-        const float* const* q = h.f32.VdV;
+        float* const* w = h.f32.Wh;
         k_mom2face3<float, const float*, float><<<grid_plane(cells, 128), 128, 0, st>>>(
-            L, h.f32.volume, q[0], q[1], q[2], o, rv[2], rv[0], rv[1]);
+            L, h.f32.volume, w[1], w[2], w[3], o, rv[2], rv[0], rv[1]);
     } else {
         Vf9<double> o;
         for (int x = 0; x < 3; ++x) { o.v[0][x] = h.VfE[0][x]; o.v[1][x] = h.VfE[1][x]; o.v[2][x] = h.Vf[x]; }
         k_mom2face3<double, const double*, double><<<grid_plane(cells, 128), 128, 0, st>>>(
-            L, g.volume, VdV.v[0], VdV.v[1], VdV.v[2], o, rv[2], rv[0], rv[1]);
+            L, g.volume, h.Wh[1], h.Wh[2], h.Wh[3], o, rv[2], rv[0], rv[1]);
     }
     h.launches++;
     for (int eD = 0; eD < 3; ++eD) {

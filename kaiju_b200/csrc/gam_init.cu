@@ -857,6 +857,7 @@ int init_problem(Handle& h, int ic, const BgSpec* bg, const double* icPar) {
     if (h.p.doMHD) launch_bflux2fld(h, s, st);
     launch_bcs(h, s, st);
     k_copy_state<<<nb(L.E, 256), 256, 0, st>>>(L.E, s, h.S[h.cur ^ 1]);
+    launch_b_check(h, true, true, st);
     launch_calcdt(h, s, 1, st);
     k_set_otime<<<1, 1, 0, st>>>(h.dScal);
     h.launches += 2;

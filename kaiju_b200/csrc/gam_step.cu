@@ -32,7 +32,7 @@ __global__ void k_step_begin(Scal* sc) {
 // per-face values EdgeLRs divides out at every stencil point (fields.F90:335-336): flux/max(area,TINY)
 // for the half state (reconstruction) and for the limiting state.
 struct F32FaceOut { float* hbA[3]; float* nbA[3]; };
-struct F32CellOut { float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; float* rho; float* VdV[3]; };
+struct F32CellOut { float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; };
 
 // Two consecutive face elements per thread with 16-byte loads and stores (E = P*Q*R is a multiple of 8 and
 // every plane starts 16-byte aligned), twice the bytes in flight per thread of a one-element loop; the
@@ -69,41 +69,68 @@ __global__ void k_predict_faces(long long E, Par p, GridP g, Vec3P mf, Vec3P omf
     }
 }
 
+// bFlux2Fld of the half-state face fluxes (Q + pdt (Q - oQ) / odt) of one cell, for the first steps after a state
+// came from outside (Scal::bGiven); out of line, so that the usual path keeps its registers
+__device__ __noinline__ void half_bxyz(const Lay& L, const GridP& g, const StateP& n, const StateP& o, double pdt,
+                                       double iodt, long long c, double* B) {
+    const long long up[3] = {c + 1, c + L.P, c + (long long)L.P * L.Q};
+    const double idV = 1.0 / g.volume[c];
+    double lo[3], hi[3], Div = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        const double q = n.mf[d][c], qu = n.mf[d][up[d]];
+        lo[d] = q + pdt * ((q - o.mf[d][c]) * iodt);
+        hi[d] = qu + pdt * ((qu - o.mf[d][up[d]]) * iodt);
+        Div += hi[d] - lo[d];
+    }
+    for (int x = 0; x < 3; ++x) {
+        double b = 0.0;
+        for (int d = 0; d < 3; ++d) b += hi[d] * g.xfc[d][x][up[d]] - lo[d] * g.xfc[d][x][c];
+        B[x] = (b - Div * g.xyzcc[x][c]) * idV;
+    }
+}
+
 // bFlux2Fld of the half state + PredictCell (mhdgroup.F90:492-518, 529-563) on every cell, plus the
 // BlockCon2Prim primitives of the half state and of state n used by the interface reconstruction.
-__global__ void k_predict_cells(Lay L, Par p, GridP g, StateP n, StateP o, StateP h, PrimP Wh, PrimP Wn, Vec3P VdV,
+//
+// HBM-bound, so what counts is how little it touches. bFlux2Fld is linear in the face fluxes and the half-state
+// fluxes are Q + pdt (Q - oQ) / odt, so the half-state field is the same extrapolation of the two states' Bxyz: 6
+// values where the fluxes and their moment arms are 16. Mom2Face forms volume times velocity from the volumes and
+// the half-state primitives, and the corner densities are the half-state primitive density, so neither is written
+// here; the conserved half state is written only for the Boris fluxes (gam_gpu_fetch("hgas") rebuilds it from
+// the primitives). 448 B per zone before, about 232 now: 256^3 1.08 -> 0.68 ms, 0.92 -> 0.55 with FP32 fluxes.
+__global__ void k_predict_cells(const __grid_constant__ Lay L, const __grid_constant__ Par p,
+                                const __grid_constant__ GridP g, const __grid_constant__ StateP n,
+                                const __grid_constant__ StateP o, StateP h, PrimP Wh, PrimP Wn,
                                 F32CellOut f, const Scal* sc) {
     Reg r = {0, L.Ni, 0, L.Nj, 0, L.Nk};
     int i, j, k;
     if (!reg_plane(r, i, j, k)) return;
     long long c = L.at(i, j, k);
-    double B[3] = {0.0, 0.0, 0.0};
     const bool f32 = f.Wh[0] != nullptr;
-    cellBxyz(L, g, h.mf, c, B);
-    if (!f32) { h.b[0][c] = B[0]; h.b[1][c] = B[1]; h.b[2][c] = B[2]; }
-    double Q[5], oQ[5], W[5], oW[5], pW[5], pQ[5];
+    const double pdt = sc->pdt, iodt = 1.0 / sc->odt;
+    double Q[5], oQ[5], W[5], oW[5], pW[5], pQ[5], B[3] = {0.0, 0.0, 0.0}, nB[3];
 #pragma unroll
     for (int v = 0; v < 5; ++v) { Q[v] = n.gas[v][c]; oQ[v] = o.gas[v][c]; }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) nB[x] = n.b[x][c];
+    if (p.doMHD) {
+        if (sc->bGiven) half_bxyz(L, g, n, o, pdt, iodt, c, B);
+        else {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) B[x] = nB[x] + pdt * ((nB[x] - o.b[x][c]) * iodt);
+        }
+    }
     cellC2P(p, oQ, oW);
     cellC2P(p, Q, W);
-    double pdt = sc->pdt, iodt = 1.0 / sc->odt;
 #pragma unroll
     for (int v = 0; v < 5; ++v) { double dQ = (W[v] - oW[v]) * iodt; pW[v] = W[v] + pdt * dQ; }
     pW[0] = dmax(pW[0], p.dFloor);
     pW[4] = dmax(pW[4], p.pFloor);
     cellP2C(p, pW, pQ);
-    // the FP32-flux path keeps the half state as floats only; the double gas half state feeds its
-    // Boris flux correction
-    if (!f32 || p.doBoris) {
+    // the conserved half state feeds the Boris flux correction
+    if (p.doBoris) {
 #pragma unroll
         for (int v = 0; v < 5; ++v) h.gas[v][c] = pQ[v];
-    }
-    // Mom2Face summand VolB*MomB/max(DenB,dFloor) (fields.F90:265-271), a pointwise cell value
-    {
-        double vol = g.volume[c], iden = 1.0 / dmax(pQ[0], p.dFloor);
-        double v0 = vol * pQ[1] * iden, v1 = vol * pQ[2] * iden, v2 = vol * pQ[3] * iden;
-        if (f32) { f.VdV[0][c] = float(v0); f.VdV[1][c] = float(v1); f.VdV[2][c] = float(v2); }
-        else { VdV.v[0][c] = v0; VdV.v[1][c] = v1; VdV.v[2][c] = v2; }
     }
     double w[5];
     if (f32) {   // FP32-flux path: float copies of every stencil input
@@ -114,16 +141,43 @@ __global__ void k_predict_cells(Lay L, Par p, GridP g, StateP n, StateP o, State
 #pragma unroll
         for (int v = 0; v < 5; ++v) f.Wn[v][c] = float(w[v]);
 #pragma unroll
-        for (int x = 0; x < 3; ++x) { f.hb[x][c] = float(B[x]); f.nb[x][c] = float(n.b[x][c]); }
-        f.rho[c] = float(pQ[0]);
+        for (int x = 0; x < 3; ++x) { f.hb[x][c] = float(B[x]); f.nb[x][c] = float(nB[x]); }
         return;
     }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) h.b[x][c] = B[x];
     blockC2P(p, pQ, w);
 #pragma unroll
     for (int v = 0; v < 5; ++v) Wh.w[v][c] = w[v];
     blockC2P(p, Q, w);
 #pragma unroll
     for (int v = 0; v < 5; ++v) Wn.w[v][c] = w[v];
+}
+// the conserved half state from its primitives (FP64 without Boris, for inspection)
+__global__ void k_half_con(Lay L, Par p, PrimP Wh, StateP h) {
+    int i, j, k;
+    if (!reg_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, i, j, k)) return;
+    const long long c = L.at(i, j, k);
+    double w[5], U[5];
+    for (int v = 0; v < 5; ++v) w[v] = Wh.w[v][c];
+    cellP2C(p, w, U);
+    for (int v = 0; v < 5; ++v) h.gas[v][c] = U[v];
+}
+// Scal::bGiven after a state came from outside: `steps`, raised by k_b_check for a state whose Bxyz is not, bit for
+// bit, what a step leaves: bFlux2Fld of its fluxes, with the cells across the axis taking their conjugates'
+// (RingFlux2FieldFix). A restart's Bxyz is, so it goes on exactly as the run it was taken from.
+__global__ void k_b_given(Scal* sc, int steps) { sc->bGiven = steps; }
+__global__ void k_b_check(Lay L, Par p, GridP g, StateP s, int steps, Scal* sc) {
+    int i, j, k;
+    if (!reg_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, i, j, k)) return;
+    int jp = j, kp = k;
+    if (p.doRing && ((p.ringDoS && j < L.js()) || (p.ringDoE && j > L.je()))) lfmCC(L, p.ringDoS, p.ringDoE, j, k, jp, kp);
+    double B[3];
+    cellBxyz(L, g, s.mf, L.at(i, jp, kp), B);
+    const long long c = L.at(i, j, k);
+    bool same = true;
+    for (int x = 0; x < 3; ++x) same = same && __double_as_longlong(B[x]) == __double_as_longlong(s.b[x][c]);
+    if (!same && sc->bGiven < steps) atomicMax(&sc->bGiven, steps);
 }
 
 // Flux2Deltas (stress.F90:150-196); O is the flux storage type (float on the FP32-flux path), the sums
@@ -435,6 +489,7 @@ __global__ void k_dt_finalize(Par p, Scal* sc, int mode) {
         sc->time = sc->time + sc->dt;
         sc->ts = sc->ts + 1;
         sc->t = sc->t + sc->dt;
+        if (sc->bGiven > 0) sc->bGiven--;
     }
     if (p.fixedTimestep) { sc->status = 0; return; }
     double dtOld = sc->dt;
@@ -726,6 +781,27 @@ GridP Handle::gridP() const {
 
 static const int TPB = 128;
 
+void mark_b_given(Handle& h, cudaStream_t st) {
+    h.hScal->bGiven = B_GIVEN_STEPS;   // set_scalars uploads the host's copy
+    k_b_given<<<1, 1, 0, st>>>(h.dScal, B_GIVEN_STEPS);
+    h.launches++;
+}
+void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st) {
+    const dim3 grid = grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB);
+    k_b_given<<<1, 1, 0, st>>>(h.dScal, 0);
+    h.launches++;
+    if (!h.p.doMHD) return;   // no fluxes to follow
+    if (n) { k_b_check<<<grid, TPB, 0, st>>>(h.L, h.p, h.gridP(), h.S[h.cur], B_GIVEN_STEPS, h.dScal); h.launches++; }
+    if (o) { k_b_check<<<grid, TPB, 0, st>>>(h.L, h.p, h.gridP(), h.S[h.cur ^ 1], 1, h.dScal); h.launches++; }
+}
+
+void launch_half_con(Handle& h, cudaStream_t st) {
+    PrimP Wh;
+    for (int v = 0; v < 5; ++v) Wh.w[v] = h.Wh[v];
+    k_half_con<<<grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB), TPB, 0, st>>>(h.L, h.p, Wh, h.H);
+    h.launches++;
+}
+
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st) {
     k_bflux2fld<<<grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB), TPB, 0, st>>>(h.L, h.gridP(), s);
     h.launches++;
@@ -784,7 +860,7 @@ void refresh_f32_background(Handle& h) {
 int ensure_f32(Handle& h) {
     if (h.f32pool) return 0;
     const long long E = h.L.E;
-    const int nplanes = 29 + 24 + 64 + 6 + (h.p.doBackground ? 18 : 0);   // 6: the I and J edges' face velocities
+    const int nplanes = 25 + 24 + 64 + 6 + (h.p.doBackground ? 18 : 0);   // 6: the I and J edges' face velocities
     if (cudaMalloc(&h.f32pool, sizeof(float) * E * nplanes) != cudaSuccess) return 3;
     cudaMemsetAsync(h.f32pool, 0, sizeof(float) * E * nplanes, h.stream);
     float* q = h.f32pool;
@@ -798,8 +874,6 @@ int ensure_f32(Handle& h) {
     for (int x = 0; x < 3; ++x) f.nbA[x] = take();
     for (int x = 0; x < 3; ++x) f.Vf[x] = take();
     for (int e = 0; e < 2; ++e) for (int x = 0; x < 3; ++x) f.VfE[e][x] = take();
-    f.rho = take();
-    for (int x = 0; x < 3; ++x) f.VdV[x] = take();
     for (int d = 0; d < 3; ++d) {
         for (int v = 0; v < 5; ++v) f.gflx[d][v] = take();
         for (int x = 0; x < 3; ++x) f.mflx[d][x] = take();
@@ -882,14 +956,12 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     }
     PrimP Wh, Wn;
     for (int v = 0; v < 5; ++v) { Wh.w[v] = h.Wh[v]; Wn.w[v] = h.Wn[v]; }
-    Vec3P VdV = {{h.VdV[0], h.VdV[1], h.VdV[2]}};
     F32CellOut fc{};
     if (h.prec == PREC_FP32FLUX) {
         for (int v = 0; v < 5; ++v) { fc.Wh[v] = h.f32.Wh[v]; fc.Wn[v] = h.f32.Wn[v]; }
-        for (int x = 0; x < 3; ++x) { fc.hb[x] = h.f32.hb[x]; fc.nb[x] = h.f32.nb[x]; fc.VdV[x] = h.f32.VdV[x]; }
-        fc.rho = h.f32.rho;
+        for (int x = 0; x < 3; ++x) { fc.hb[x] = h.f32.hb[x]; fc.nb[x] = h.f32.nb[x]; }
     }
-    k_predict_cells<<<grid_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, TPB), TPB, 0, st>>>(L, p, g, nS, oS, h.H, Wh, Wn, VdV, fc, h.dScal);
+    k_predict_cells<<<grid_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, TPB), TPB, 0, st>>>(L, p, g, nS, oS, h.H, Wh, Wn, fc, h.dScal);
     h.launches += 2;
     if (p.doRing) launch_ring_bfix(h, h.H, st, h.prec == PREC_FP32FLUX);   // bFlux2Fld's ring fix
     if (p.predFixLFM) launch_predfix_lfm(h, h.H, st, h.prec == PREC_FP32FLUX);   // HackPredictor

@@ -13,9 +13,8 @@ enum Prec { PREC_FP64 = 0, PREC_FP32FLUX = 1 };
 // float copies used by the FP32-flux path: stencil inputs written by the predictor each step and
 // metric planes converted once
 struct F32Planes {
-    float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; float* hbA[3]; float* nbA[3]; float* Vf[3]; float* rho;
+    float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; float* hbA[3]; float* nbA[3]; float* Vf[3];
     float* VfE[2][3];   // face velocities for the I and J edges (Vf: the K edges')
-    float* VdV[3];
     float* gflx[3][5]; float* mflx[3][3];   // area-scaled interface fluxes
     float* volume; float* face[3]; float* edge[3]; float* Tf[3][9]; float* Te[3][6]; float* Teb[3][4];
     // background field: fcB0, bFlux0/face and edgB0 (only with a background)
@@ -49,7 +48,6 @@ struct Handle {
     double* Wh[5];        // primitives of the half state (BlockCon2Prim), for reconstruction
     double* Wn[5];        // primitives of state n, for the limiter
     double* E[3];         // Efld (edge-centred, times edge length)
-    double* VdV[3];       // half-state volume * momentum / max(rho, dFloor) per cell (Mom2Face summand)
     double* hbA[3];       // half-state face flux / max(face area, TINY) (EdgeLRs reconstruction values)
     double* nbA[3];       // limiter-state face flux / max(face area, TINY) (EdgeLRs limiter values)
     double* Vf[3];        // face velocities pushed along dT1 for the K edges (the last direction, as the reference leaves it)
@@ -108,6 +106,12 @@ void launch_dt_finalize(Handle& h, int mode, cudaStream_t st);
 enum { PH_PREDICT = 0, PH_EFIELD, PH_FLUXES, PH_DELTAS, PH_UPDATE, PH_DT, PH_BCS, NPHASE };
 // Kernels used outside the step
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st);
+// Scal::bGiven after State n and/or oState came from outside the step: set to its most, or found by checking the
+// states named (the other is known to be bFlux2Fld of its fluxes)
+void mark_b_given(Handle& h, cudaStream_t st);
+void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st);
+// h.H.gas from the half-state primitives, which the FP64 step without Boris does not write
+void launch_half_con(Handle& h, cudaStream_t st);
 // withB: ghost B copied with the gas (set-up); a step leaves it to the bFlux2Fld of the ghost cells that follows
 void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB = true);
 void launch_calcdt(Handle& h, const StateP& s, int mode, cudaStream_t st);   // mode 0: in-step, 1: initial (no time advance)

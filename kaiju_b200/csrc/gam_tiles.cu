@@ -372,6 +372,7 @@ int gam_tiles_create(gam_tiles_t** out, gam_gpu_t* const* tiles, int n, int peri
     fan(T, [&](int q) { enqueue_fill(T, q, 0, true, true); });
     fan(T, [&](int q) {
         Handle& h = H(T, q);
+        mark_b_given(h, h.stream);
         k_red_reset<<<1, 1, 0, h.stream>>>(h.dScal);
         launch_calcdt_partial(h, h.S[h.cur], h.stream);
     });
@@ -576,6 +577,8 @@ int gam_gpu_halo_unpack(gam_gpu_t* G, int side, unsigned what, const void* src) 
             i += len;
         }
     launch_chunks(h, tab, h.stream);
+    // a step's own halo fill (State, before step_ghosts) is followed by the halo's bFlux2Fld; any other is not
+    if (h.tilePhase != 2 || what != GAM_HALO_STATE) mark_b_given(h, h.stream);
     return cudaGetLastError() == cudaSuccess ? GAM_OK : GAM_ERR_CUDA;
 }
 
