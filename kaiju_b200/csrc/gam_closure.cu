@@ -358,11 +358,18 @@ __global__ void k_loss_w(Lay L, const float* corr, const float* res, const float
     }
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
-__global__ void k_loss_sum(const float* part, int nblk, double* acc) {
-    if (threadIdx.x != 0) return;
+// one block of 256: one thread that added the 1024 partials in turn took 27 us, now 3.6
+__global__ void __launch_bounds__(256) k_loss_sum(const float* part, int nblk, double* acc) {
+    __shared__ double red[256];
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[b];
-    acc[0] += s;
+    for (int b = threadIdx.x; b < nblk; b += 256) s += part[b];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) acc[0] += red[0];
 }
 
 // output gradient: dL/dy for the lower d-face of each active cell = fluxScale * A * (w(cell) - w(cell below)),
@@ -626,6 +633,7 @@ int gam_closure_create(gam_closure_t** out, int Nip, int Njp, int Nkp, unsigned 
             cudaMalloc(&C->wbwd[l], sizeof(__nv_bfloat16) * 27 * bc * 32))
             return fail(GAM_ERR_CUDA);
     }
+    if (net_clear_weights(C->wfwd, C->wbwd, C->stream) != 0) return fail(GAM_ERR_CUDA);
     // channels-last activations: act (16 + 3*32), pre (3*32), grad (4*32) bf16 per cell; out (24) fp32 planes
     const long long E = L.E;
     const long long bfPerCell = NET_IN_PITCH + 3 * NET_PITCH + 3 * NET_PITCH + 4 * NET_PITCH;
@@ -929,12 +937,12 @@ static int closure_sample_pass(gam_closure* C, int slot, bool train, float lr) {
     if (C->lossMode == GAM_CLOSURE_LOSS_FACE) {
         k_loss_face<<<nb, 256, 0, C->stream>>>(L, C->nb.out, C->sFace[slot], C->geom, n,
                                                train ? C->nb.grad[NET_LAYERS - 1] : nullptr, C->lossPart);
-        k_loss_sum<<<1, 32, 0, C->stream>>>(C->lossPart, nb, C->lossAcc);
+        k_loss_sum<<<1, 256, 0, C->stream>>>(C->lossPart, nb, C->lossAcc);
     } else {
         k_closure_corr<<<grid_plane(Reg{L.is(), L.Nip + 1, L.js(), L.Njp + 1, L.ks(), L.Nkp + 1}, 256), 256, 0,
                          C->stream>>>(L, C->nb.out, n, C->geom, C->corr);
         k_loss_w<<<nb, 256, 0, C->stream>>>(L, C->corr, C->sRes[slot], C->geom, n, C->sDt[slot], C->wts, C->lossPart);
-        k_loss_sum<<<1, 32, 0, C->stream>>>(C->lossPart, nb, C->lossAcc);
+        k_loss_sum<<<1, 256, 0, C->stream>>>(C->lossPart, nb, C->lossAcc);
     }
     if (train) {
         if (C->lossMode != GAM_CLOSURE_LOSS_FACE)
@@ -989,12 +997,12 @@ int gam_closure_eval(gam_closure_t* C, const int* slots, int n, double* loss, do
             } else if (C->lossMode == GAM_CLOSURE_LOSS_FACE) {   // no correction: the targets alone
                 k_loss_face<<<1024, 256, 0, C->stream>>>(L, nullptr, C->sFace[slots[q]], C->geom, nrm, nullptr,
                                                          C->lossPart);
-                k_loss_sum<<<1, 32, 0, C->stream>>>(C->lossPart, 1024, C->lossAcc);
+                k_loss_sum<<<1, 256, 0, C->stream>>>(C->lossPart, 1024, C->lossAcc);
             } else {   // no correction: the residual alone
                 CKC(cudaMemsetAsync(C->corr, 0, sizeof(float) * L.E * NET_OUT, C->stream));
                 k_loss_w<<<1024, 256, 0, C->stream>>>(L, C->corr, C->sRes[slots[q]], C->geom, nrm, C->sDt[slots[q]],
                                                        C->wts, C->lossPart);
-                k_loss_sum<<<1, 32, 0, C->stream>>>(C->lossPart, 1024, C->lossAcc);
+                k_loss_sum<<<1, 256, 0, C->stream>>>(C->lossPart, 1024, C->lossAcc);
             }
         }
         double a[2];

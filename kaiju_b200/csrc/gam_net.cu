@@ -4,20 +4,16 @@
 
 #include "gam_net.cuh"
 #include "gam_tc.cuh"
+#include "gam_tma.cuh"
 
 namespace gam {
 namespace {
 
 constexpr uint32_t WAIT_LIMIT = 1u << 24;   // mbarrier polls before a wait gives up (well above any MMA time)
 
-__device__ __forceinline__ float bf2f(__nv_bfloat16 x) { return __bfloat162float(x); }
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_d(float x) {
     return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
-}
-__host__ __device__ __forceinline__ long long tap_off(int t, int P, int Q) {
-    int di = t % 3 - 1, dj = (t / 3) % 3 - 1, dk = t / 9 - 1;
-    return (long long)di + (long long)P * (dj + (long long)Q * dk);
 }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);   // a at the lower address
@@ -27,7 +23,6 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 enum { MODE_HIDDEN = 0, MODE_OUT = 1, MODE_BWD = 2 };
 
 struct ConvArgs {
-    const __nv_bfloat16* x;    // input activations, channels-last with pitch CINP
     const __nv_bfloat16* gz;   // MODE_BWD: pre-activation of the previous layer (pitch 32): the epilogue
                                // multiplies the input gradient by its GELU derivative
     const __nv_bfloat16* w;    // packed weights, 27 taps of [32 x CINP] K-major blocks
@@ -40,19 +35,19 @@ struct ConvArgs {
     int* err;
 };
 
+constexpr int ROWS = 128;        // cells of a window: the M of a tile
+constexpr int TILE = ROWS - 2;   // output cells of a tile (its first and last rows only feed their neighbours)
+
 template <int CINP>
 struct ConvShape {
-    static constexpr int COUTP = 32;
-    static constexpr int ROWS = 130;                   // 128 cells and one on each side (di = -1, +1)
-    static constexpr int KCH = CINP / 8;               // 16-byte channel chunks per cell
-    static constexpr int LBO = ROWS * 16;              // bytes between the channel-chunk blocks of a window
-    static constexpr int WIN = KCH * LBO;
-    static constexpr int TAPB = COUTP * CINP * 2;      // one tap's packed weights
+    static constexpr int WIN = ROWS * CINP * 2;        // a window: 128 cells x CINP channels, swizzled rows
+    static constexpr int TAPB = 32 * CINP * 2;         // one tap's packed weights
     static constexpr int WB = (27 * TAPB + 1023) / 1024 * 1024;   // all taps, resident for the CTA's life
-    static constexpr int STAGE = (WIN + 127) / 128 * 128;
-    static constexpr int NS = 5;                       // window stages in the ring
-    static constexpr int BYTES = WB + NS * STAGE + 1024;
-    static constexpr int THREADS = 160;                // 4 worker warps (copies, epilogue) + 1 MMA warp
+    static constexpr int NS = CINP == 32 ? 5 : 12;     // window stages in the ring
+    // two CTAs per SM, no more: each holds 256 of the SM's 512 TMEM columns
+    static constexpr int BYTES = WB + NS * WIN + 1024;
+    static constexpr int THREADS = 192;                // 4 epilogue warps, 1 MMA warp, 1 copy warp
+    static_assert(2 * (BYTES + 4096) <= 227 * 1024 && 3 * BYTES > 227 * 1024, "two CTAs per SM");
 };
 
 __device__ __forceinline__ unsigned char* align1k(unsigned char* p) {
@@ -60,74 +55,103 @@ __device__ __forceinline__ unsigned char* align1k(unsigned char* p) {
     return p + ((1024u - (s & 1023u)) & 1023u);
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(tc::smem_u32(dst)), "l"(src), "r"(bytes)
-                 : "memory");
-}
-// arrive on the mbarrier once every cp.async this thread issued so far has landed
-__device__ __forceinline__ void cp_async_arrive(uint64_t* mbar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(tc::smem_u32(mbar)) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" :: "r"(tc::smem_u32(mbar))
                  : "memory");
 }
+__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// out[cell][n] = sum over taps t and input channels c of in[cell + off(t)][c] * W_t[n][c], 128 cells per tile.
-// The weights of all 27 taps stay in shared memory. Warps 0-3 copy windows into a ring of NS stages (full[s] completes when the 128 threads' copies of a
-// window have landed) and run the epilogue of each finished tile (warp w reads TMEM lanes 32w..32w+31);
-// one thread of warp 4 issues the MMAs of a window once its stage is full and commits them to empty[s]
-// (the stage may be refilled) and, after a tile's last window, to tfull[a] (accumulator a is ready).
-// Two TMEM accumulators alternate between tiles; tempty[a] completes when the workers have read one.
+// out[c][n] = sum over the 27 taps t and input channels k of in[c + off(t)][k] * W_t[n][k].
+//
+// The three taps di = -1, 0, +1 of a (dj, dk) pair read the same cells, one row apart. One MMA takes all three at
+// once, N = 96 output columns: D[r][di * 32 + n] = sum over (dj, dk), k of in[cell(r) + off(dj, dk)][k] * W[n][k], and
+// the epilogue adds out[c] = D[c-1][di=-1] + D[c][di=0] + D[c+1][di=+1] (a lane shuffle, and a row each side of a warp
+// through shared memory). The A operand is then read from shared memory once instead of three times -- with N = 32
+// that read, not the math, set the MMA's time -- and it needs no shifted start, so a window is a plain 128 x CINP box
+// that one tensor copy brings in swizzled, with no copy instructions in the other warps. What is left is the copies'
+// row rate: the 16- and the 32-channel layers, with half and twice the bytes and MMAs, take almost the same time.
+// Warps 0-3: epilogue (warp w reads TMEM lanes 32w..32w+31). One thread of warp 4 issues the MMAs of a window once
+// full[s] completes, commits them to empty[s] and, after a tile's last window, to tfull[a]; one thread of warp 5 fills
+// the ring of NS windows. Two TMEM accumulators alternate; tempty[a] completes when the epilogue has read one.
+// 128^3 (137 x 137 x 144 cells): 32 -> 32 channels 533 -> 291 us, 32 -> 27 514 -> 256, 16 -> 32 317 -> 261, against
+// per-thread 16-byte copies, N = 32 and the epilogue in the copying warps.
 template <int CINP, int MODE>
-__global__ void __launch_bounds__(160) k_conv(ConvArgs a) {
+__global__ void __launch_bounds__(192, 2) k_conv(const __grid_constant__ CUtensorMap xmap, ConvArgs a) {
     using S = ConvShape<CINP>;
-    static_assert(CINP % 16 == 0, "K step");
     extern __shared__ unsigned char smraw[];
     unsigned char* sW = align1k(smraw);
     unsigned char* sStage = sW + S::WB;
     __shared__ __align__(8) uint64_t full[S::NS], empty[S::NS], tfull[2], tempty[2], wready;
+    __shared__ __align__(16) float edge[2][4][2][32];   // [tile parity][warp]: last row's di=-1, first row's di=+1
     __shared__ uint32_t tmemBase;
     __shared__ int failed;
     __shared__ float sBias[32];
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // the bias, once per CTA: the epilogue reads it from shared memory instead of 32 global loads per tile
     if (tid < 32) sBias[tid] = (MODE != MODE_BWD && tid < a.cout) ? a.bias[tid] : 0.f;
     if (tid == 0) {
-        for (int q = 0; q < S::NS; ++q) { tc::mbar_init(&full[q], 128); tc::mbar_init(&empty[q], 1); }
+        for (int q = 0; q < S::NS; ++q) { tc::mbar_init(&full[q], 1); tc::mbar_init(&empty[q], 1); }
         for (int q = 0; q < 2; ++q) { tc::mbar_init(&tfull[q], 1); tc::mbar_init(&tempty[q], 128); }
-        tc::mbar_init(&wready, 128);
+        tc::mbar_init(&wready, 1);
         failed = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tma::fence_barrier_init();
     }
-    if (warp == 0) tc::tmem_alloc(&tmemBase, 64);
+    if (warp == 0) tc::tmem_alloc(&tmemBase, 256);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tbase = tmemBase;
 
-    const long long ntiles = (a.c1 - a.c0 + 127) / 128;
+    const long long ntiles = (a.c1 - a.c0 + TILE - 1) / TILE;
     const long long myTiles = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    auto firstCell = [&](long long T) { return a.c0 + (blockIdx.x + T * (long long)gridDim.x) * TILE - 1; };
 
     if (warp < 4) {
-        // ---------------- workers: copies and epilogues
-        auto epilogue = [&](long long T) -> bool {
+        // ---------------- epilogues
+        bool ok = true;
+        for (long long T = 0; T < myTiles; ++T) {
             const int acc = (int)(T & 1);
-            if (!tc::mbar_wait(&tfull[acc], (uint32_t)((T >> 1) & 1), WAIT_LIMIT)) return false;
-            tc::fence_after_sync();
-            float v[32];
-            tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + acc * 32, v);
+            // a warp whose wait gave up still meets the others at the barrier of every tile
+            ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(&tfull[acc], (uint32_t)((T >> 1) & 1), WAIT_LIMIT));
+            const uint32_t t0 = tbase + ((uint32_t)(warp * 32) << 16) + acc * 128;
+            float v[32], d[32];
+            if (ok) {
+                tc::fence_after_sync();
+                tc::tmem_ld32(t0, d);   // di = -1: from the row before
+                if (lane == 31)
+#pragma unroll
+                    for (int q = 0; q < 32; q += 4)
+                        *reinterpret_cast<float4*>(&edge[acc][warp][0][q]) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
+#pragma unroll
+                for (int q = 0; q < 32; ++q) v[q] = __shfl_up_sync(0xffffffffu, d[q], 1);
+                tc::tmem_ld32(t0 + 64, d);   // di = +1: from the row after
+                if (lane == 0)
+#pragma unroll
+                    for (int q = 0; q < 32; q += 4)
+                        *reinterpret_cast<float4*>(&edge[acc][warp][1][q]) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
+            }
+            epi_barrier();
+            if (!ok) continue;
+            if (lane == 0 && warp > 0)
+#pragma unroll
+                for (int q = 0; q < 32; ++q) v[q] = edge[acc][warp - 1][0][q];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+                const float up = __shfl_down_sync(0xffffffffu, d[q], 1);
+                v[q] += lane == 31 && warp < 3 ? edge[acc][warp + 1][1][q] : up;
+            }
+            tc::tmem_ld32(t0 + 32, d);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] += d[q];
             tc::fence_before_sync();
             mbar_arrive(&tempty[acc]);
-            const long long cell = a.c0 + (blockIdx.x + T * (long long)gridDim.x) * 128 + tid;
-            if (cell >= a.c1) return true;
+            const long long cell = firstCell(T) + tid;
+            if (tid == 0 || tid == ROWS - 1 || cell >= a.c1) continue;
             if (MODE == MODE_OUT) {
 #pragma unroll
                 for (int co = 0; co < 32; ++co)
                     if (co < a.cout) a.yf[(long long)co * a.E + cell] = v[co] + sBias[co];
-                return true;
+                continue;
             }
             uint32_t py[16], pz[16];
             if (MODE == MODE_BWD) {
@@ -161,40 +185,13 @@ __global__ void __launch_bounds__(160) k_conv(ConvArgs a) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) z4[q] = make_uint4(pz[4 * q], pz[4 * q + 1], pz[4 * q + 2], pz[4 * q + 3]);
             }
-            return true;
-        };
-        // the weights of all taps, once
-        for (int id = tid; id < 27 * S::TAPB / 16; id += 128)
-            cp_async16(sW + id * 16, reinterpret_cast<const unsigned char*>(a.w) + id * 16, 16u);
-        cp_async_arrive(&wready);
-        bool ok = true;
-        for (long long T = 0; T < myTiles && ok; ++T) {
-            const long long cell0 = a.c0 + (blockIdx.x + T * (long long)gridDim.x) * 128;
-            for (int w = 0; w < 9 && ok; ++w) {
-                const long long it = T * 9 + w;
-                const int st = (int)(it % S::NS);
-                const long long use = it / S::NS;
-                if (use > 0 && !tc::mbar_wait(&empty[st], (uint32_t)((use - 1) & 1), WAIT_LIMIT)) { ok = false; break; }
-                const int dj = w % 3 - 1, dk = w / 3 - 1;
-                const long long base = cell0 - 1 + (long long)a.P * (dj + (long long)a.Q * dk);
-                unsigned char* dst = sStage + st * S::STAGE;
-                for (int id = tid; id < S::ROWS * S::KCH; id += 128) {
-                    const int row = id / S::KCH, kc = id % S::KCH;
-                    const long long cell = base + row;
-                    const bool inb = cell >= 0 && cell < a.E;
-                    cp_async16(dst + kc * S::LBO + row * 16, a.x + (inb ? cell : 0) * CINP + kc * 8, inb ? 16u : 0u);
-                }
-                cp_async_arrive(&full[st]);
-            }
-            if (ok && T > 0) ok = epilogue(T - 1);
         }
-        if (ok && myTiles > 0) ok = epilogue(myTiles - 1);
         if (!ok) failed = 1;
-        cp_async_wait_all();
     } else if (tid == 128) {
         // ---------------- MMA issue
-        const uint32_t idesc = tc::idesc_bf16_f32(128, S::COUTP);
+        const uint32_t idesc = tc::idesc_bf16_f32(128, 96);
         constexpr uint32_t SBO_W = CINP / 8 * 128;
+        constexpr uint32_t SWZ = CINP == 32 ? tc::SWZ_64B : tc::SWZ_32B, SBO_X = 8 * CINP * 2;
         long long issued = 0;   // windows whose MMAs were committed
         bool ok = myTiles == 0 || tc::mbar_wait(&wready, 0u, WAIT_LIMIT);
         for (long long T = 0; T < myTiles && ok; ++T) {
@@ -204,18 +201,14 @@ __global__ void __launch_bounds__(160) k_conv(ConvArgs a) {
                 const long long it = T * 9 + w;
                 const int st = (int)(it % S::NS);
                 if (!tc::mbar_wait(&full[st], (uint32_t)((it / S::NS) & 1), WAIT_LIMIT)) { ok = false; break; }
-                tc::fence_smem_async();   // the generic-proxy copies, to the tensor core
                 tc::fence_after_sync();
-                const uint32_t win = tc::smem_u32(sStage + st * S::STAGE);
-                const uint32_t wt = tc::smem_u32(sW) + (3 * (w % 3) + 9 * (w / 3)) * S::TAPB;   // taps of (dj, dk)
+                const uint32_t win = tc::smem_u32(sStage + st * S::WIN);
+                const uint32_t wt = tc::smem_u32(sW) + 3 * w * S::TAPB;   // the taps di = -1, 0, 1 of (dj, dk), 96 rows
 #pragma unroll
-                for (int di = -1; di <= 1; ++di) {
-#pragma unroll
-                    for (int ks = 0; ks < CINP / 16; ++ks) {
-                        const uint64_t ad = tc::desc_kmajor(win + (di + 1) * 16 + ks * 2 * S::LBO, S::LBO, 128);
-                        const uint64_t bd = tc::desc_kmajor(wt + (di + 1) * S::TAPB + ks * 256, 128, SBO_W);
-                        tc::mma_bf16(tbase + acc * 32, ad, bd, idesc, !(w == 0 && di == -1 && ks == 0));
-                    }
+                for (int ks = 0; ks < CINP / 16; ++ks) {
+                    const uint64_t ad = tc::desc_swz(win + ks * 32, 16, SBO_X, SWZ);
+                    const uint64_t bd = tc::desc_kmajor(wt + ks * 256, 128, SBO_W);
+                    tc::mma_bf16(tbase + acc * 128, ad, bd, idesc, !(w == 0 && ks == 0));
                 }
                 tc::mma_commit(&empty[st]);
                 if (w == 8) tc::mma_commit(&tfull[acc]);
@@ -230,198 +223,231 @@ __global__ void __launch_bounds__(160) k_conv(ConvArgs a) {
                 tc::mbar_wait(&empty[(int)(it % S::NS)], (uint32_t)((it / S::NS) & 1), WAIT_LIMIT);
             }
         }
+    } else if (tid == 160 && myTiles > 0) {
+        // ---------------- copies
+        tma::arrive_expect_tx(&wready, 27 * S::TAPB);
+        tma::load_bulk(sW, a.w, 27 * S::TAPB, &wready);
+        bool ok = true;
+        long long it = 0;
+        for (long long T = 0; T < myTiles && ok; ++T) {
+            const long long row0 = firstCell(T);
+            for (int w = 0; w < 9; ++w, ++it) {
+                const int st = (int)(it % S::NS);
+                if (it >= S::NS && !tc::mbar_wait(&empty[st], (uint32_t)((it / S::NS - 1) & 1), WAIT_LIMIT)) { ok = false; break; }
+                tma::arrive_expect_tx(&full[st], S::WIN);
+                tma::load2(sStage + st * S::WIN, &xmap, 0,
+                           (int)(row0 + (long long)a.P * ((w % 3 - 1) + (long long)a.Q * (w / 3 - 1))), &full[st]);
+            }
+        }
+        if (!ok) failed = 1;
+        // the copies in flight land before the CTA's shared memory goes, whatever became of the other warps
+        tc::mbar_wait(&wready, 0u, WAIT_LIMIT);
+        for (long long q = it > S::NS ? it - S::NS : 0; q < it; ++q)
+            tc::mbar_wait(&full[(int)(q % S::NS)], (uint32_t)((q / S::NS) & 1), WAIT_LIMIT);
     }
     tc::fence_before_sync();
     __syncthreads();
     if (tid == 0 && failed) atomicExch(a.err, 1);
-    if (warp == 0) tc::tmem_free(tbase, 64);
+    if (warp == 0) tc::tmem_free(tbase, 256);
 }
 
 // ------------------------------------------------------------------ weight gradient
 struct DwArgs {
-    const __nv_bfloat16* x;    // layer input activations, channels-last with pitch CINP
-    const __nv_bfloat16* dy;   // gradient w.r.t. the layer's pre-activation, channels-last pitch 32
-    float* partial;            // [gridDim.x][NG][128][COUTP]
+    float* partial;            // [gridDim.x][NG][128][96]
     long long E, c0, c1;
-    int P, Q, cin, cout;
+    int P, Q, cin;
     int* err;
 };
 
-template <int CINP, int COUTP>
+template <int CINP>
 struct DwShape {
-    static constexpr int G = 128 / CINP;                  // taps per 128-row group
-    static constexpr int NG = (27 + G - 1) / G;
-    static constexpr int AB = 128 * 16 * 2;               // one group's A: 128 rows x 16 cells
-    static constexpr int BB = COUTP * 16 * 2;
-    static constexpr int STAGE = (NG * AB + BB + 1023) / 1024 * 1024;
-    static constexpr int COLS = NG * COUTP <= 32 ? 32 : NG * COUTP <= 64 ? 64 : NG * COUTP <= 128 ? 128 : 256;
-    // request enough shared memory that TMEM (512 columns per SM) always covers the resident CTAs
-    static constexpr int BYTES_MIN = 2 * STAGE + 1024;
-    static constexpr int PER_SM = 512 / COLS;
-    static constexpr int BYTES = BYTES_MIN > (228 * 1024 / PER_SM - 2048) ? BYTES_MIN : (228 * 1024 / PER_SM - 2048);
+    static constexpr int XWIN = ROWS * CINP * 2;          // a window of the layer's input: 128 cells x CINP
+    static constexpr int GWIN = ROWS * 32 * 2;            // a window of the gradient: 128 cells x 32
+    static constexpr int G = 128 / CINP;                  // windows (dj, dk) per group of 128 rows
+    static constexpr int NG = (9 + G - 1) / G;
+    static constexpr int STAGE = 9 * XWIN + 3 * GWIN;
+    static constexpr int NS = CINP == 32 ? 2 : 3;
+    static constexpr int COLS = NG * 96 <= 256 ? 256 : 512;
+    // the last group's rows beyond the ninth window read what follows it (their results are not used)
+    static constexpr int SLACK = NG * G * XWIN > STAGE ? NG * G * XWIN - STAGE : 0;
+    static constexpr int BYTES = NS * STAGE + SLACK + 1024;
+    static_assert(STAGE % 1024 == 0 && BYTES <= 226 * 1024 && 2 * BYTES > 227 * 1024, "one CTA per SM");
 };
 
-// D[(tap, ci)][co] = sum over cells of x[ci][cell + off(tap)] * dy'[co][cell], 16 cells per MMA
-template <int CINP, int COUTP>
-__global__ void __launch_bounds__(128) k_conv_dw(DwArgs a) {
-    using S = DwShape<CINP, COUTP>;
+// dW[t][co][ci] = sum over cells c of x[c + off(t)][ci] * dy[c][co]. With c' = c + di the three taps of a (dj, dk)
+// pair share x[c' + off(dj, dk)] and shift dy instead, so a tile of 128 cells c' takes 9 windows of x and 3 of dy, and
+// one MMA contracts 16 of its cells for 4 (or 8) windows' channels (M = 128) against 3 shifts x 32 output channels
+// (N = 96). Both operands are MN-major: the rows that a tensor copy brings in are the contraction index, and nothing is
+// transposed or copied by threads. A CTA accumulates all its tiles in TMEM and writes one partial; a fixed-order sum
+// follows. Cells outside [c0, c1) have a zero gradient, so the tiles need no masks.
+// Building A with 2-byte loads (one per element and tap) took 153 us per 32-channel layer at 32^3; now 17.3.
+template <int CINP>
+__global__ void __launch_bounds__(192, 1) k_conv_dw(const __grid_constant__ CUtensorMap xmap,
+                                                    const __grid_constant__ CUtensorMap gmap, DwArgs a) {
+    using S = DwShape<CINP>;
     extern __shared__ unsigned char smraw[];
     unsigned char* sbase = align1k(smraw);
-    __shared__ __align__(8) uint64_t mbar[2];
+    __shared__ __align__(8) uint64_t full[S::NS], empty[S::NS], done;
     __shared__ uint32_t tmemBase;
+    __shared__ int failed;
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
-        tc::mbar_init(&mbar[0], 1);
-        tc::mbar_init(&mbar[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int q = 0; q < S::NS; ++q) { tc::mbar_init(&full[q], 1); tc::mbar_init(&empty[q], 1); }
+        tc::mbar_init(&done, 1);
+        failed = 0;
+        tma::fence_barrier_init();
     }
     if (warp == 0) tc::tmem_alloc(&tmemBase, S::COLS);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tbase = tmemBase;
-    const uint32_t idesc = tc::idesc_bf16_f32(128, COUTP);
-    const unsigned short* xs = reinterpret_cast<const unsigned short*>(a.x);
-
-    uint32_t use0 = 0, use1 = 0;
-    int ok = 1, it = 0;
-    const long long nsteps = (a.c1 - a.c0 + 15) / 16;
-    for (long long s = blockIdx.x; s < nsteps; s += gridDim.x, ++it) {
-        const long long cell0 = a.c0 + s * 16;
-        const int b = it & 1;
-        const uint32_t use = b ? use1 : use0;
-        bool fine = true;
-        if (use > 0) fine = tc::mbar_wait(&mbar[b], (use - 1) & 1u, WAIT_LIMIT);
-        unsigned char* st = sbase + b * S::STAGE;
-        if (fine) {
-            // A: row m = tid of every group: x[ci][cell0 + k + off(tap)] for k = 0..15
-            const int ci = tid % CINP;
-#pragma unroll 1
-            for (int g = 0; g < S::NG; ++g) {
-                const int t = g * S::G + tid / CINP;
-                uint32_t pk[8];
-                const bool live = t < 27 && ci < a.cin;
-                const long long c0 = cell0 + (live ? tap_off(t, a.P, a.Q) : 0);
-#pragma unroll
-                for (int k = 0; k < 16; k += 2) {
-                    const long long c = c0 + k;
-                    uint32_t lo = (live && c >= 0 && c < a.E) ? xs[c * CINP + ci] : 0u;
-                    uint32_t hi = (live && c + 1 >= 0 && c + 1 < a.E) ? xs[(c + 1) * CINP + ci] : 0u;
-                    pk[k / 2] = lo | (hi << 16);
-                }
-                unsigned char* dA = st + g * S::AB;
-                *reinterpret_cast<uint4*>(dA + tc::kmajor_off(tid, 0, 16)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *reinterpret_cast<uint4*>(dA + tc::kmajor_off(tid, 8, 16)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            }
-            // B: row n = output channel, 16 cells of the gradient w.r.t. the pre-activation
-            if (tid < COUTP * 2) {
-                const int n = tid >> 1, h = tid & 1;
-                const unsigned short* dys = reinterpret_cast<const unsigned short*>(a.dy);
-                uint32_t pk[4];
-#pragma unroll
-                for (int k = 0; k < 8; k += 2) {
-                    const long long c = cell0 + h * 8 + k;
-                    uint32_t lo = (n < a.cout && c < a.c1) ? dys[c * NET_PITCH + n] : 0u;
-                    uint32_t hi = (n < a.cout && c + 1 < a.c1) ? dys[(c + 1) * NET_PITCH + n] : 0u;
-                    pk[k / 2] = lo | (hi << 16);
-                }
-                *reinterpret_cast<uint4*>(st + S::NG * S::AB + tc::kmajor_off(n, h * 8, 16)) =
-                    make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            }
-        }
-        tc::fence_smem_async();
-        if (!__syncthreads_and(fine)) { ok = 0; break; }
-        if (tid == 0) {
+    const long long ntiles = (a.c1 - a.c0 + 2 + ROWS - 1) / ROWS;   // c' in [c0 - 1, c1 + 1)
+    const long long myTiles = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    if (tid == 128) {
+        const uint32_t idesc = tc::idesc_bf16_f32_mn(128, 96);
+        constexpr uint32_t SWZ = CINP == 32 ? tc::SWZ_64B : tc::SWZ_32B, XROW = CINP * 2;
+        bool ok = true;
+        long long T = 0;
+        for (; T < myTiles; ++T) {
+            const int st = (int)(T % S::NS);
+            if (!tc::mbar_wait(&full[st], (uint32_t)((T / S::NS) & 1), WAIT_LIMIT)) { ok = false; break; }
             tc::fence_after_sync();
-            const uint64_t bd = tc::desc_kmajor(tc::smem_u32(st + S::NG * S::AB), 128, 256);
-#pragma unroll 1
-            for (int g = 0; g < S::NG; ++g) {
-                const uint64_t ad = tc::desc_kmajor(tc::smem_u32(st + g * S::AB), 128, 256);
-                tc::mma_bf16(tbase + g * COUTP, ad, bd, idesc, it > 0);
-            }
-            tc::mma_commit(&mbar[b]);
-        }
-        if (b) ++use1; else ++use0;
-    }
-    if (ok && it > 0) {
-        const int bl = (it - 1) & 1;
-        const uint32_t ul = bl ? use1 : use0;
-        bool fine = tc::mbar_wait(&mbar[bl], (ul - 1) & 1u, WAIT_LIMIT);
-        ok = __syncthreads_and(fine);
-    }
-    float* part = a.partial + (long long)blockIdx.x * S::NG * 128 * COUTP;
-    if (ok) {
-        tc::fence_after_sync();
-#pragma unroll 1
-        for (int g = 0; g < S::NG; ++g) {
-            float acc[32];
-            if (it > 0) tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + g * COUTP, acc);
-            else for (int q = 0; q < 32; ++q) acc[q] = 0.f;
-            float* row = part + ((long long)g * 128 + tid) * COUTP;
+            const uint32_t xw = tc::smem_u32(sbase + st * S::STAGE), gw = xw + 9 * S::XWIN;
+            for (int ks = 0; ks < ROWS / 16; ++ks) {
+                const uint64_t bd = tc::desc_swz(gw + ks * 16 * 64, S::GWIN, 8 * 64, tc::SWZ_64B);
 #pragma unroll
-            for (int n = 0; n < COUTP; ++n) row[n] = acc[n];
+                for (int g = 0; g < S::NG; ++g)
+                    tc::mma_bf16(tbase + g * 96,
+                                 tc::desc_swz(xw + g * S::G * S::XWIN + ks * 16 * XROW, S::XWIN, 8 * XROW, SWZ), bd, idesc,
+                                 T > 0 || ks > 0);
+            }
+            tc::mma_commit(&empty[st]);
         }
-    } else {
-        if (tid == 0) atomicExch(a.err, 1);
-        if (use0) tc::mbar_wait(&mbar[0], (use0 - 1) & 1u, WAIT_LIMIT);
-        if (use1) tc::mbar_wait(&mbar[1], (use1 - 1) & 1u, WAIT_LIMIT);
+        if (ok) tc::mma_commit(&done);
+        else {
+            failed = 1;
+            if (T > 0) tc::mbar_wait(&empty[(int)((T - 1) % S::NS)], (uint32_t)(((T - 1) / S::NS) & 1), WAIT_LIMIT);
+        }
+    } else if (tid == 160) {
+        bool ok = true;
+        long long T = 0;
+        for (; T < myTiles; ++T) {
+            const int st = (int)(T % S::NS);
+            if (T >= S::NS && !tc::mbar_wait(&empty[st], (uint32_t)((T / S::NS - 1) & 1), WAIT_LIMIT)) { ok = false; break; }
+            const long long row0 = a.c0 - 1 + (blockIdx.x + T * (long long)gridDim.x) * ROWS;
+            unsigned char* dst = sbase + st * S::STAGE;
+            tma::arrive_expect_tx(&full[st], S::STAGE);
+            for (int w = 0; w < 9; ++w)
+                tma::load2(dst + w * S::XWIN, &xmap, 0,
+                           (int)(row0 + (long long)a.P * ((w % 3 - 1) + (long long)a.Q * (w / 3 - 1))), &full[st]);
+            for (int di = -1; di <= 1; ++di)
+                tma::load2(dst + 9 * S::XWIN + (di + 1) * S::GWIN, &gmap, 0, (int)(row0 - di), &full[st]);
+        }
+        if (!ok) failed = 1;
+        for (long long q = T > S::NS ? T - S::NS : 0; q < T; ++q)
+            tc::mbar_wait(&full[(int)(q % S::NS)], (uint32_t)((q / S::NS) & 1), WAIT_LIMIT);
+    } else if (warp < 4 && myTiles > 0) {
+        if (tc::mbar_wait(&done, 0u, WAIT_LIMIT)) {
+            tc::fence_after_sync();
+            float* part = a.partial + (long long)blockIdx.x * S::NG * 128 * 96;
+#pragma unroll 1
+            for (int q = 0; q < S::NG * 3; ++q) {
+                const int g = q / 3, b = q % 3;
+                float acc[32];
+                tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + g * 96 + b * 32, acc);
+                if (g * S::G + tid / CINP < 9 && tid % CINP < a.cin) {
+                    float4* row = reinterpret_cast<float4*>(part + ((long long)g * 128 + tid) * 96 + b * 32);
+#pragma unroll
+                    for (int n = 0; n < 8; ++n) row[n] = make_float4(acc[4 * n], acc[4 * n + 1], acc[4 * n + 2], acc[4 * n + 3]);
+                }
+            }
+            tc::fence_before_sync();
+        } else failed = 1;
     }
-    tc::fence_before_sync();
     __syncthreads();
+    if (tid == 0 && failed) atomicExch(a.err, 1);
     if (warp == 0) tc::tmem_free(tbase, S::COLS);
 }
 
-// grads W[t][co][ci] of one layer = the fixed-order sum of the CTAs' partials
-template <int CINP, int COUTP>
-__global__ void k_dw_reduce(const float* partial, int nblk, float* gW, int cin, int cout) {
-    using S = DwShape<CINP, COUTP>;
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= 27 * cout * cin) return;
-    const int ci = id % cin, co = (id / cin) % cout, t = id / (cin * cout);
-    const int g = t / S::G, m = (t % S::G) * CINP + ci;
+// grads W[t][co][ci] of one layer = the fixed-order sum of the CTAs' partials: a block per (window, input channel),
+// 96 columns (shift, output channel) by 8 slices of the CTAs
+template <int CINP>
+__global__ void __launch_bounds__(768) k_dw_reduce(const float* partial, int nblk, float* gW, int cin, int cout) {
+    using S = DwShape<CINP>;
+    __shared__ double red[8][96];
+    const int w = blockIdx.x / cin, ci = blockIdx.x % cin, col = threadIdx.x % 96, sl = threadIdx.x / 96;
+    const float* q = partial + ((long long)(w / S::G) * 128 + (w % S::G) * CINP + ci) * 96 + col;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += partial[(((long long)b * S::NG + g) * 128 + m) * COUTP + co];
-    gW[id] = (float)s;
+#pragma unroll 4
+    for (int b = sl; b < nblk; b += 8) s += q[(long long)b * S::NG * 128 * 96];
+    red[sl][col] = s;
+    __syncthreads();
+    const int co = col % 32;
+    if (sl != 0 || co >= cout) return;
+    for (int r = 1; r < 8; ++r) s += red[r][col];
+    gW[((long long)(3 * w + col / 32) * cout + co) * cin + ci] = (float)s;
 }
 
-// bias gradient: per-block partial sums of the gradient w.r.t. the pre-activation over the cell range, then
-// a fixed-order sum
-__global__ void k_bias_partial(const __nv_bfloat16* dy, long long c0, long long c1, int cout, float* part) {
-    __shared__ float red[256];
-    for (int co = 0; co < cout; ++co) {
-        float s = 0.f;
-        for (long long c = c0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; c < c1;
-             c += (long long)gridDim.x * blockDim.x)
-            s += bf2f(dy[c * NET_PITCH + co]);
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-            __syncthreads();
+// bias gradient: per-block partial sums of the gradient w.r.t. the pre-activation over the cell range, then a
+// fixed-order sum. A thread reads 8 channels of a cell at once (one channel after the other over the whole range,
+// 2 bytes at a time, took 27 us at 32^3, and the final sum by one thread per channel 19 us; now 5.6 and 4.0).
+__global__ void __launch_bounds__(256) k_bias_partial(const __nv_bfloat16* dy, long long c0, long long c1, float* part) {
+    __shared__ float red[8][32];
+    const int tid = threadIdx.x, q = tid & 3;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (long long c = c0 + blockIdx.x * 64LL + (tid >> 2); c < c1; c += gridDim.x * 64LL) {
+        const uint4 u = *reinterpret_cast<const uint4*>(dy + c * NET_PITCH + q * 8);
+        const uint32_t r[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&r[e]);
+            s[2 * e] += __low2float(h);
+            s[2 * e + 1] += __high2float(h);
         }
-        if (threadIdx.x == 0) part[(long long)blockIdx.x * cout + co] = red[0];
-        __syncthreads();
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        for (int o = 4; o < 32; o <<= 1) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+        if ((tid & 31) < 4) red[tid >> 5][q * 8 + e] = s[e];
+    }
+    __syncthreads();
+    if (tid < 32) {
+        float t = 0.f;
+        for (int w = 0; w < 8; ++w) t += red[w][tid];
+        part[blockIdx.x * 32 + tid] = t;
     }
 }
-__global__ void k_bias_reduce(const float* part, int nblk, int cout, float* gb) {
-    const int co = threadIdx.x;
-    if (co >= cout) return;
+__global__ void __launch_bounds__(1024) k_bias_reduce(const float* part, int nblk, int cout, float* gb) {
+    __shared__ double red[32][33];
+    const int co = threadIdx.x & 31, r = threadIdx.x >> 5;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[(long long)b * cout + co];
+    for (int b = r; b < nblk; b += 32) s += part[b * 32 + co];
+    red[r][co] = s;
+    __syncthreads();
+    if (r != 0 || co >= cout) return;
+    for (int q = 1; q < 32; ++q) s += red[q][co];
     gb[co] = (float)s;
 }
 
 // ------------------------------------------------------------------ packing and Adam
-// forward blocks: tap t, row n = output channel, K = input channel; backward-data blocks: tap 26 - t
-// (the mirrored offset), row n = input channel, K = output channel
-__global__ void k_pack(const float* W, int cin, int cout, __nv_bfloat16* fwd, int fCinP, int fCoutP,
-                       __nv_bfloat16* bwd, int bCinP, int bCoutP) {
+// forward blocks: tap t, row n = output channel, K = input channel; backward-data blocks: tap 26 - t (the mirrored
+// offset), row n = input channel, K = output channel. All layers in one launch (blockIdx.y); the padding rows and
+// channels are zeroed once, when the blocks are allocated (net_clear_weights), and never written.
+struct PackArgs {
+    const float* W[NET_LAYERS];
+    __nv_bfloat16 *fwd[NET_LAYERS], *bwd[NET_LAYERS];
+    int cin[NET_LAYERS], cout[NET_LAYERS];
+};
+__global__ void k_pack(const __grid_constant__ PackArgs a) {
+    const int l = blockIdx.y, cin = a.cin[l], cout = a.cout[l];
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= 27 * cout * cin) return;
+    const int fCinP = (cin + 15) / 16 * 16, bCinP = (cout + 15) / 16 * 16;
     const int ci = id % cin, co = (id / cin) % cout, t = id / (cin * cout);
-    const __nv_bfloat16 w = __float2bfloat16_rn(W[id]);
-    fwd[((long long)t * fCoutP * fCinP * 2 + tc::kmajor_off(co, ci, fCinP)) / 2] = w;
-    if (bwd) bwd[((long long)(26 - t) * bCoutP * bCinP * 2 + tc::kmajor_off(ci, co, bCinP)) / 2] = w;
+    const __nv_bfloat16 w = __float2bfloat16_rn(a.W[l][id]);
+    a.fwd[l][((long long)t * 32 * fCinP * 2 + tc::kmajor_off(co, ci, fCinP)) / 2] = w;
+    if (a.bwd[l]) a.bwd[l][((long long)(26 - t) * 32 * bCinP * 2 + tc::kmajor_off(ci, co, bCinP)) / 2] = w;
 }
 
 __global__ void k_adam(float* p, const float* g, float* m, float* v, long long n, float lr, float b1, float b2,
@@ -455,13 +481,16 @@ int sm_count() {
 }
 
 template <int CINP, int MODE>
-void launch_conv(const ConvArgs& a, cudaStream_t st) {
+int launch_conv(const __nv_bfloat16* x, const ConvArgs& a, cudaStream_t st) {
     using S = ConvShape<CINP>;
-    long long ntiles = (a.c1 - a.c0 + 127) / 128;
-    long long grid = sm_count() * (CINP == 16 ? 4 : 2);
+    CUtensorMap xmap;
+    if (!tma::act_map(&xmap, x, CINP, a.E, ROWS)) return (int)cudaErrorInvalidValue;
+    const long long ntiles = (a.c1 - a.c0 + TILE - 1) / TILE;
+    long long grid = sm_count() * 2;
     if (grid > ntiles) grid = ntiles;
     if (grid < 1) grid = 1;
-    k_conv<CINP, MODE><<<(unsigned)grid, S::THREADS, S::BYTES, st>>>(a);
+    k_conv<CINP, MODE><<<(unsigned)grid, S::THREADS, S::BYTES, st>>>(xmap, a);
+    return 0;
 }
 
 }  // namespace
@@ -472,30 +501,41 @@ int net_init() {
     set_smem(k_conv<32, MODE_HIDDEN>, ConvShape<32>::BYTES);
     set_smem(k_conv<32, MODE_OUT>, ConvShape<32>::BYTES);
     set_smem(k_conv<32, MODE_BWD>, ConvShape<32>::BYTES);
-    set_smem(k_conv_dw<16, 32>, DwShape<16, 32>::BYTES);
-    set_smem(k_conv_dw<32, 32>, DwShape<32, 32>::BYTES);
+    set_smem(k_conv_dw<16>, DwShape<16>::BYTES);
+    set_smem(k_conv_dw<32>, DwShape<32>::BYTES);
     sm_count();
     return (int)cudaGetLastError();
 }
 
-int net_dw_blocks() { return sm_count() * 2; }
+int net_dw_blocks() { return sm_count(); }
 long long net_partial_floats(int nblocks) {
-    // the largest layer: CINP 32 -> 7 groups of 128 x 32
-    return (long long)nblocks * 7 * 128 * 32;
+    // the largest layer: CINP 32 -> 3 groups of 128 x 96
+    return (long long)nblocks * DwShape<32>::NG * 128 * 96;
 }
 size_t net_act_bytes(long long E) { return (size_t)E * sizeof(__nv_bfloat16); }
+
+int net_clear_weights(__nv_bfloat16* wfwd[NET_LAYERS], __nv_bfloat16* wbwd[NET_LAYERS], cudaStream_t st) {
+    NetShape s = net_shape();
+    for (int l = 0; l < NET_LAYERS; ++l) {
+        cudaMemsetAsync(wfwd[l], 0, sizeof(__nv_bfloat16) * 27 * pad16(s.cin[l]) * 32, st);
+        if (wbwd[l]) cudaMemsetAsync(wbwd[l], 0, sizeof(__nv_bfloat16) * 27 * pad16(s.cout[l]) * 32, st);
+    }
+    return (int)cudaGetLastError();
+}
 
 int net_pack_weights(const float* params, __nv_bfloat16* wfwd[NET_LAYERS], __nv_bfloat16* wbwd[NET_LAYERS],
                      cudaStream_t st) {
     NetShape s = net_shape();
+    PackArgs a{};
+    int most = 0;
     for (int l = 0; l < NET_LAYERS; ++l) {
-        const int fCinP = pad16(s.cin[l]), fCoutP = 32, bCinP = pad16(s.cout[l]), bCoutP = 32;
-        cudaMemsetAsync(wfwd[l], 0, sizeof(__nv_bfloat16) * 27 * fCinP * fCoutP, st);
-        if (wbwd[l]) cudaMemsetAsync(wbwd[l], 0, sizeof(__nv_bfloat16) * 27 * bCinP * bCoutP, st);
+        a.W[l] = params + net_param_offset(l);
+        a.fwd[l] = wfwd[l]; a.bwd[l] = wbwd[l];
+        a.cin[l] = s.cin[l]; a.cout[l] = s.cout[l];
         const int n = 27 * s.cin[l] * s.cout[l];
-        k_pack<<<(n + 255) / 256, 256, 0, st>>>(params + net_param_offset(l), s.cin[l], s.cout[l], wfwd[l], fCinP,
-                                                fCoutP, wbwd[l], bCinP, bCoutP);
+        if (n > most) most = n;
     }
+    k_pack<<<dim3((most + 255) / 256, NET_LAYERS), 256, 0, st>>>(a);
     return (int)cudaGetLastError();
 }
 
@@ -504,31 +544,38 @@ int net_forward(const NetBox& b, __nv_bfloat16* const wfwd[NET_LAYERS], const fl
     NetShape s = net_shape();
     for (int l = 0; l < NET_LAYERS; ++l) {
         ConvArgs a{};
-        a.x = nb.act[l];
         a.w = wfwd[l];
         a.bias = params + net_param_offset(l) + 27LL * s.cout[l] * s.cin[l];
         a.E = b.E; a.c0 = b.c0; a.c1 = b.c1; a.P = b.P; a.Q = b.Q;
         a.cout = s.cout[l];
         a.err = err;
+        int rc;
         if (l < NET_LAYERS - 1) {
             a.y = nb.act[l + 1];
             a.z = keepPre ? nb.pre[l] : nullptr;
-            if (l == 0) launch_conv<16, MODE_HIDDEN>(a, st);
-            else launch_conv<32, MODE_HIDDEN>(a, st);
+            if (l == 0) rc = launch_conv<16, MODE_HIDDEN>(nb.act[l], a, st);
+            else rc = launch_conv<32, MODE_HIDDEN>(nb.act[l], a, st);
         } else {
             a.yf = nb.out;
-            launch_conv<32, MODE_OUT>(a, st);
+            rc = launch_conv<32, MODE_OUT>(nb.act[l], a, st);
         }
+        if (rc) return rc;
     }
     return (int)cudaGetLastError();
 }
 
-template <int CINP, int COUTP>
-static void launch_dw(const DwArgs& a, int nblk, float* gW, cudaStream_t st) {
-    using S = DwShape<CINP, COUTP>;
-    k_conv_dw<CINP, COUTP><<<nblk, 128, S::BYTES, st>>>(a);
-    const int n = 27 * a.cin * a.cout;
-    k_dw_reduce<CINP, COUTP><<<(n + 255) / 256, 256, 0, st>>>(a.partial, nblk, gW, a.cin, a.cout);
+template <int CINP>
+static int launch_dw(const __nv_bfloat16* x, const __nv_bfloat16* dy, const DwArgs& a, int nblk, float* gW, int cout,
+                     cudaStream_t st) {
+    using S = DwShape<CINP>;
+    CUtensorMap xmap, gmap;
+    if (!tma::act_map(&xmap, x, CINP, a.E, ROWS) || !tma::act_map(&gmap, dy, NET_PITCH, a.E, ROWS))
+        return (int)cudaErrorInvalidValue;
+    const long long ntiles = (a.c1 - a.c0 + 2 + ROWS - 1) / ROWS;
+    const int grid = ntiles < nblk ? (int)ntiles : nblk;
+    k_conv_dw<CINP><<<grid, 192, S::BYTES, st>>>(xmap, gmap, a);
+    k_dw_reduce<CINP><<<9 * a.cin, 768, 0, st>>>(a.partial, grid, gW, a.cin, cout);
+    return 0;
 }
 
 // gradients of every parameter from the output gradient nb.grad[3] (channels-last, pitch 32), given the
@@ -539,20 +586,22 @@ int net_backward(const NetBox& b, __nv_bfloat16* const wbwd[NET_LAYERS], NetBuff
     const int nblk = net_dw_blocks();
     for (int l = NET_LAYERS - 1; l >= 0; --l) {
         DwArgs d{};
-        d.x = nb.act[l]; d.dy = nb.grad[l]; d.partial = nb.partial;
-        d.E = b.E; d.c0 = b.c0; d.c1 = b.c1; d.P = b.P; d.Q = b.Q; d.cin = s.cin[l]; d.cout = s.cout[l]; d.err = err;
+        d.partial = nb.partial;
+        d.E = b.E; d.c0 = b.c0; d.c1 = b.c1; d.P = b.P; d.Q = b.Q; d.cin = s.cin[l]; d.err = err;
         float* gW = grads + net_param_offset(l);
-        if (l == 0) launch_dw<16, 32>(d, nblk, gW, st);
-        else launch_dw<32, 32>(d, nblk, gW, st);
-        k_bias_partial<<<nblk, 256, 0, st>>>(nb.grad[l], b.c0, b.c1, s.cout[l], nb.partial);
-        k_bias_reduce<<<1, 32, 0, st>>>(nb.partial, nblk, s.cout[l], gW + 27LL * s.cout[l] * s.cin[l]);
+        int rc = l == 0 ? launch_dw<16>(nb.act[l], nb.grad[l], d, nblk, gW, s.cout[l], st)
+                        : launch_dw<32>(nb.act[l], nb.grad[l], d, nblk, gW, s.cout[l], st);
+        if (rc) return rc;
+        k_bias_partial<<<nblk, 256, 0, st>>>(nb.grad[l], b.c0, b.c1, nb.partial);
+        k_bias_reduce<<<1, 1024, 0, st>>>(nb.partial, nblk, s.cout[l], gW + 27LL * s.cout[l] * s.cin[l]);
         if (l > 0) {   // gradient w.r.t. the previous layer's pre-activation: through this layer, then GELU'
             ConvArgs a{};
-            a.x = nb.grad[l]; a.gz = nb.pre[l - 1]; a.w = wbwd[l];
+            a.gz = nb.pre[l - 1]; a.w = wbwd[l];
             a.y = nb.grad[l - 1];
             a.E = b.E; a.c0 = b.c0; a.c1 = b.c1; a.P = b.P; a.Q = b.Q;
             a.cout = s.cin[l]; a.err = err;
-            launch_conv<32, MODE_BWD>(a, st);
+            rc = launch_conv<32, MODE_BWD>(nb.grad[l], a, st);
+            if (rc) return rc;
         }
     }
     return (int)cudaGetLastError();

@@ -9,14 +9,12 @@
 //   GELU between layers.
 //
 // Every convolution is an implicit GEMM on the tensor cores (tcgen05.mma kind::f16, BF16 x BF16 -> FP32
-// in TMEM): a CTA owns 128 consecutive cells (M = 128) and all output channels (N = 32). For each of the
-// 9 (dj, dk) offsets it copies (cp.async, 16-byte chunks) a window of 130 cells x input channels into
-// shared memory, one block of rows per channel chunk with the rows 16 bytes apart, so the A operand of
-// the three taps di = -1, 0, +1 is the same window read from row 0, 1 or 2 (a 16-byte shift of the
-// descriptor's start address). Windows are triple-buffered: the copy of window w+2 overlaps the MMAs of
-// window w. The weight gradient contracts over cells instead (M = 128 rows of (tap, input channel),
-// N = output channels, K = 16 cells per MMA), each CTA accumulating all taps in TMEM over its cells and
-// writing one partial that a fixed-order reduction sums.
+// in TMEM): a CTA owns 128 consecutive cells (M = 128) and, for each of the 9 (dj, dk) offsets, multiplies a window of
+// 128 cells x input channels (one tensor copy, swizzled) by the weights of the three taps di = -1, 0, +1 at once
+// (N = 96); the epilogue adds the three results of neighbouring rows. The weight gradient contracts over cells instead
+// (M = 128 rows of (window, input channel), N = 3 shifts x 32 output channels, K = 16 cells per MMA, both operands
+// MN-major), each CTA accumulating all taps in TMEM over its cells and writing one partial that a fixed-order
+// reduction sums.
 #pragma once
 #include <cuda_bf16.h>
 #include <cstdint>
@@ -70,6 +68,7 @@ struct NetBuffers {
 };
 
 // host launchers (gam_net.cu); each returns 0 or a CUDA error code
+int net_clear_weights(__nv_bfloat16* wfwd[NET_LAYERS], __nv_bfloat16* wbwd[NET_LAYERS], cudaStream_t st);
 int net_pack_weights(const float* params, __nv_bfloat16* wfwd[NET_LAYERS], __nv_bfloat16* wbwd[NET_LAYERS],
                      cudaStream_t st);
 int net_forward(const NetBox& b, __nv_bfloat16* const wfwd[NET_LAYERS], const float* params, NetBuffers& nb,

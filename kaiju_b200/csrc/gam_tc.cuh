@@ -28,6 +28,15 @@ __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr, uint32_t lbo, ui
     return d;                 // base offset 0, legacy LBO mode, layout type 0 (no swizzle)
 }
 
+// Swizzled operands as tensor copies leave them (rows of 32 or 64 bytes, the copy's swizzle of the same span). K-major:
+// a row holds K (32-byte span: 16 elements, 64-byte: 32) and 8-row groups are sbo bytes apart. MN-major: a row is one
+// K index and its span is a block of 16 or 32 consecutive M (or N) elements; blocks are lbo bytes apart, groups of 8
+// K rows sbo bytes. The swizzle works on address bits, so a K step inside a K-major span only advances saddr by 32.
+enum { SWZ_64B = 4, SWZ_32B = 6 };
+__device__ __forceinline__ uint64_t desc_swz(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t swz) {
+    return desc_kmajor(saddr, lbo, sbo) | (uint64_t)swz << 61;
+}
+
 // instruction descriptor: kind::f16 with BF16 A and B (both K-major), FP32 D, dense, M x N
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
     return (1u << 4)                       // D format F32
@@ -35,6 +44,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          | (1u << 10)                      // B format BF16
          | ((uint32_t)(N >> 3) << 17)      // N / 8
          | ((uint32_t)(M >> 4) << 24);     // M / 16
+}
+
+// the same with both operands MN-major
+__host__ __device__ constexpr uint32_t idesc_bf16_f32_mn(int M, int N) {
+    return idesc_bf16_f32(M, N) | (1u << 15) | (1u << 16);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool acc) {

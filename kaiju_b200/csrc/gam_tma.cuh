@@ -51,6 +51,21 @@ inline bool plane_map(CUtensorMap* m, const void* plane, int esize, const Lay& L
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tensor map of a channels-last BF16 activation array (n cells of ch = 16 or 32 channels, contiguous) with a box of
+// all channels by `rows` cells, written to shared memory with the swizzle of the row's span (32 or 64 bytes); cells
+// below 0 or from n on arrive as zeros
+inline bool act_map(CUtensorMap* m, const void* base, int ch, long long n, int rows) {
+    EncodeTiledFn enc = encoder();
+    if (!enc || !base || (reinterpret_cast<uintptr_t>(base) & 15) || (ch != 16 && ch != 32)) return false;
+    cuuint64_t dim[2] = {(cuuint64_t)ch, (cuuint64_t)n};
+    cuuint64_t stride[1] = {(cuuint64_t)ch * 2};
+    cuuint32_t box[2] = {(cuuint32_t)ch, (cuuint32_t)rows};
+    cuuint32_t es[2] = {1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dim, stride, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // make an mbarrier initialisation visible to the asynchronous proxy before any copy completes on it
 __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -66,6 +81,18 @@ __device__ __forceinline__ void load3(void* dst, const CUtensorMap* map, int x, 
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         :: "r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(mbar)), "r"(x), "r"(y), "r"(z)
         : "memory");
+}
+
+__device__ __forceinline__ void load2(void* dst, const CUtensorMap* map, int x, int y, uint64_t* mbar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        :: "r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(mbar)), "r"(x), "r"(y)
+        : "memory");
+}
+// contiguous bytes (a multiple of 16, both addresses 16-byte aligned) into shared memory
+__device__ __forceinline__ void load_bulk(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(tc::smem_u32(dst)), "l"(src), "r"(bytes), "r"(tc::smem_u32(mbar)) : "memory");
 }
 
 }  // namespace tma
