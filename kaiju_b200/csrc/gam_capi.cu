@@ -199,7 +199,12 @@ int alloc_handle(gam_gpu* G, const gam_model_c* m) {
     ring_kernels_init();
     CK(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     h.ownStream = true;
-    const size_t planes = 11 * 3 + 10 + 11 + 9 + 24 + 91 + 6;   // + the I and J edges' face velocities
+    for (int q = 0; q < Handle::NSIDE; ++q) {
+        CK(cudaStreamCreateWithFlags(&h.side[q], cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&h.joinEv[q], cudaEventDisableTiming));
+    }
+    CK(cudaEventCreateWithFlags(&h.forkEv, cudaEventDisableTiming));
+    const size_t planes = 11 * 3 + 10 + 11 + 9 + 24 + 92 + 6;   // + the I and J edges' face velocities
     h.poolPlanes = planes;
     CK(cudaMalloc(&h.pool, sizeof(double) * L.E * planes));
     CK(cudaMemsetAsync(h.pool, 0, sizeof(double) * L.E * planes, h.stream));
@@ -227,7 +232,7 @@ int alloc_handle(gam_gpu* G, const gam_model_c* m) {
     h.volume = take();
     for (int x = 0; x < 3; ++x) h.xyzcc[x] = take();
     for (int d = 0; d < 3; ++d) for (int x = 0; x < 3; ++x) h.xfc[d][x] = take();
-    h.di = take(); h.dj = take(); h.dk = take();
+    h.di = take(); h.dj = take(); h.dk = take(); h.dl = take();
     for (int d = 0; d < 3; ++d) h.face[d] = take();
     for (int d = 0; d < 3; ++d) h.edge[d] = take();
     for (int d = 0; d < 3; ++d) for (int c = 0; c < 9; ++c) h.Tf[d][c] = take();
@@ -386,6 +391,7 @@ int gam_gpu_create(gam_gpu_t** out, const gam_model_c* m, const gam_grid_c* g, c
     if (!rc) rc = h2d_planes(G, &h.di, 1, g->di, ce);
     if (!rc) rc = h2d_planes(G, &h.dj, 1, g->dj, ce);
     if (!rc) rc = h2d_planes(G, &h.dk, 1, g->dk, ce);
+    if (!rc) launch_min_length(h, h.stream);
     if (!rc) rc = h2d_planes(G, h.face, 3, g->face, fe);
     if (!rc) rc = h2d_planes(G, h.edge, 3, g->edge, fe);
     if (!rc) { for (int d = 0; d < 3; ++d) for (int c = 0; c < 9; ++c) pl[d * 9 + c] = h.Tf[d][c]; rc = h2d_planes(G, pl, 27, g->Tf, fe); }
@@ -847,6 +853,11 @@ void gam_gpu_destroy(gam_gpu_t* G) {
     if (G->copyStream) cudaStreamDestroy(G->copyStream);
     if (h.dScal) cudaFree(h.dScal);
     if (h.hScal) cudaFreeHost(h.hScal);
+    for (int q = 0; q < Handle::NSIDE; ++q) {
+        if (h.side[q]) cudaStreamDestroy(h.side[q]);
+        if (h.joinEv[q]) cudaEventDestroy(h.joinEv[q]);
+    }
+    if (h.forkEv) cudaEventDestroy(h.forkEv);
     if (h.stream && h.ownStream) cudaStreamDestroy(h.stream);
     if (h.msphpool) cudaFree(h.msphpool);
     delete G;
@@ -940,7 +951,9 @@ int ens_capture(gam_ensemble* E, int flip, cudaGraphExec_t* out) {
             if (!E->active[m]) continue;
             Handle& h = E->members[m]->h;
             cudaStreamWaitEvent(h.stream, E->fork, 0);
+            h.alone = false;
             if (step_enqueue(h, h.cur ^ flip, nullptr, false, parts[pi]) != 0) rc = GAM_ERR_CUDA;
+            h.alone = true;
             cudaEventRecord(E->join[m], h.stream);
             cudaStreamWaitEvent(E->root, E->join[m], 0);
         }

@@ -75,7 +75,6 @@ constexpr unsigned int STAGE_DRAIN = 1u << 28;
 // Time-dependent scalars kept on the device so a whole step can be captured and replayed.
 struct Scal {
     double t, dt, dt0, time, otime;   // Model%t, Model%dt, Model%dt0, State%time, oState%time
-    double pdt, odt;                  // predictor half-step and state separation of this step
     unsigned long long dtMinBits;     // running min of CellDT (bit pattern of a non-negative double)
     unsigned int nanCount;            // cells whose CellDT was NaN
     int ts;
@@ -91,6 +90,7 @@ struct Scal {
     // learned closure: 1 when this step's corrected update failed positivity and the plain fluxes were used
     int closureReject;
     int closureRejects;               // steps that fell back, since the handle was created
+    unsigned int blocksDone;          // CalcDT blocks that have taken part in the minimum so far
     // nonzero once a kernel's bounded wait on its own asynchronous copies gave up (the step's results are
     // not valid); CalcDT reports it as status bit 8
     unsigned int waitFail;
@@ -107,7 +107,7 @@ struct GridP {
     const double* volume;
     const double* xyzcc[3];
     const double* xfc[3][3];   // [dir][xyz]
-    const double* di; const double* dj; const double* dk;
+    const double* dl;          // CellDT's length: the least of di, dj, dk
     const double* face[3];
     const double* edge[3];
     const double* Tf[3][9];    // [dir][component]

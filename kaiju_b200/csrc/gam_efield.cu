@@ -155,9 +155,11 @@ void efield_kernels_init() {
     efield_kernels_init_f32();
 }
 
-// CalcElecField (fields.F90:70-232): E = 0, then for eD = I, J, K: Mom2Face along dT1, EMF on the edges
-void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st) {
+// CalcElecField (fields.F90:70-232): E = 0, then for eD = I, J, K: Mom2Face along dT1, EMF on the edges (the three
+// directions beside one another)
+void enqueue_efield(Handle& h, const StateP& nS, Branches& br) {
     (void)nS;   // the limiter values come from the precomputed nbA planes
+    cudaStream_t st = br.st;
     const Lay& L = h.L;
     // E = 0 (fields.F90:88) needs no pass per step: the edge kernels rewrite the same edges every step, and
     // every edge outside them stays zero from the pool's zeroing (initialisation clears its scratch use)
@@ -202,14 +204,17 @@ void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st) {
         launch_mom2face<double>(L, g.volume, h.Wh[1], h.Wh[2], h.Wh[3], o, rv[2], rv[0], rv[1], st);
     }
     h.launches++;
-    for (int eD = 0; eD < 3; ++eD) {
+    for (int eD = 2; eD >= 0; --eD) {   // the last on st itself
+        const cudaStream_t es = eD > 0 ? br.go(SIDE_EDGE + eD - 1) : st;
         for (int x = 0; x < 3; ++x) {
             in32.Vf[x] = eD < 2 ? h.f32.VfE[eD][x] : h.f32.Vf[x];
             in64.Vf[x] = eD < 2 ? h.VfE[eD][x] : h.Vf[x];
         }
-        if (f32) launch_edge_dir_f32(h, in32, eD, re[eD], st);
-        else launch_edge_dir<double, double>(h, in64, eD, re[eD], st);
+        if (f32) launch_edge_dir_f32(h, in32, eD, re[eD], es);
+        else launch_edge_dir<double, double>(h, in64, eD, re[eD], es);
     }
+    br.join(SIDE_EDGE);
+    br.join(SIDE_EDGE + 1);
 }
 
 }  // namespace gam

@@ -30,7 +30,7 @@ static FluxSrc<float> flux_src32(Handle& h) {
     return in;
 }
 
-void enqueue_fluxes_f32(Handle& h, const StateP& nS, cudaStream_t st) {
+void enqueue_fluxes_f32(Handle& h, const StateP& nS, const cudaStream_t* st) {
     (void)nS;
     fluxes_all<float, float>(h, flux_src32(h), st);
 }

@@ -694,6 +694,7 @@ int init_grid_from_corners(Handle& h) {
     Out3 fc = {{h.face[0], h.face[1], h.face[2]}};
     k_grid_dl<<<nb(nc, 256), 256, 0, st>>>(L, h.volume, fc, h.di, h.dj, h.dk);
     if (h.p.doRing) launch_ring_grid_fix(h, st);   // init.F90:967-968, before the edge geometry
+    launch_min_length(h, st);
     for (int d = 0; d < 3; ++d) {
         int is = 0, ie = L.Ni, js = 0, je = L.Nj, ks = 0, ke = L.Nk;   // maximal bounds (corner index space)
         if (d == 0) { ie = L.Ni - 1; ks = 1; ke = L.Nk - 1; }

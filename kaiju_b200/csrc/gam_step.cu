@@ -17,14 +17,14 @@
 namespace gam {
 
 // ================================================================================ step scalars
-// AdvanceMHD trap (mhdgroup.F90:26-28) and the predictor time factors (:459)
-__global__ void k_step_begin(Scal* sc) {
-    if (fabs(sc->otime - sc->time) < TINY) sc->otime = sc->time - sc->dt;
-    sc->pdt = 0.5 * sc->dt;
-    sc->odt = sc->time - sc->otime;
-    sc->dtMinBits = 0x7FF0000000000000ull;  // +inf
-    sc->nanCount = 0u;
-    sc->closureReject = 0;
+// The predictor's time factors (mhdgroup.F90:459) with AdvanceMHD's trap (:26-28), formed by every thread that needs
+// them: a launch of their own took as long as a small problem's kernels
+struct StepTimes { double pdt, iodt; };
+__device__ __forceinline__ StepTimes step_times(const Scal* sc) {
+    const double t = sc->time, dt = sc->dt;
+    double ot = sc->otime;
+    if (fabs(ot - t) < TINY) ot = t - dt;
+    return StepTimes{0.5 * dt, 1.0 / (t - ot)};
 }
 
 // ================================================================================ predictor
@@ -41,7 +41,8 @@ __global__ void k_predict_faces(long long E, Par p, GridP g, Vec3P mf, Vec3P omf
                                 F32FaceOut o, const Scal* sc) {
     long long l = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x);
     if (l >= E) return;
-    const double pdt = sc->pdt, iodt = 1.0 / sc->odt;   // reciprocals where the reference divides repeatedly
+    const StepTimes tm = step_times(sc);
+    const double pdt = tm.pdt, iodt = tm.iodt;   // reciprocals where the reference divides repeatedly
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const double2 Q2 = *reinterpret_cast<const double2*>(mf.v[c] + l);
@@ -107,7 +108,8 @@ __global__ void k_predict_cells(const __grid_constant__ Lay L, const __grid_cons
     if (!reg_plane(r, i, j, k)) return;
     long long c = L.at(i, j, k);
     const bool f32 = f.Wh[0] != nullptr;
-    const double pdt = sc->pdt, iodt = 1.0 / sc->odt;
+    const StepTimes tm = step_times(sc);
+    const double pdt = tm.pdt, iodt = tm.iodt;
     double Q[5], oQ[5], W[5], oW[5], pW[5], pQ[5], B[3] = {0.0, 0.0, 0.0}, nB[3];
 #pragma unroll
     for (int v = 0; v < 5; ++v) { Q[v] = n.gas[v][c]; oQ[v] = o.gas[v][c]; }
@@ -423,7 +425,58 @@ __host__ __device__ inline Reg reg_dt(const Lay& L, const Par& p) {
     return r;
 }
 
-__global__ void k_calcdt(Lay L, Par p, GridP g, StateP s, Scal* sc) {
+// UpdateStateData time bookkeeping (gamapp.F90:113-114, mhdgroup.F90:104-105) and the rest of CalcDT
+// (step.F90:103-166): checks, the tFin clamp and the 10*dt0 clamp. mode 1 = initial dt (Hatch). It leaves the next
+// step's minimum, NaN count and closure flag cleared.
+__device__ __noinline__ void dt_finalize(const Par& p, Scal* sc, int mode) {
+    const unsigned long long bits = __ldcg(&sc->dtMinBits);
+    const unsigned nan = __ldcg(&sc->nanCount);
+    sc->dtMinBits = 0x7FF0000000000000ull;
+    sc->nanCount = 0u;
+    sc->closureReject = 0;
+    if (mode == 0) {
+        sc->otime = sc->time;
+        sc->time = sc->time + sc->dt;
+        sc->ts = sc->ts + 1;
+        sc->t = sc->t + sc->dt;
+        if (sc->bGiven > 0) sc->bGiven--;
+    }
+    if (p.fixedTimestep) { sc->status = 0; return; }
+    double dtOld = sc->dt;
+    double dtMin = __longlong_as_double((long long)bits);
+    if (bits >= 0x7FF0000000000000ull || dtMin > HUGEV) dtMin = HUGEV;
+    int st = 0;
+    if (dtMin == HUGEV) st |= 1;
+    if (sc->ts > 0) {
+        if (dtOld / dtMin >= 10) st |= 2;
+        if ((sc->dt0 > TINY) && (dtMin / sc->dt0 <= p.limDT0)) st |= 2;
+        if (dtMin <= TINY) st |= 1;
+    }
+    if (nan) st |= 4;
+    if (sc->waitFail) st |= 8;
+    double r = dtMin;
+    if ((sc->t + r) > p.tFin) r = dmax(p.tFin - sc->t, TINY);
+    if (sc->dt0 > TINY && r > 10.0 * sc->dt0) r = 10.0 * sc->dt0;
+    sc->dt = r;
+    sc->status = st;
+    sc->sticky |= st;
+    sc->lastNan = nan;
+    sc->waitFail = 0u;   // reported in this step's status (and the sticky OR); the next step starts clear
+}
+__global__ void k_dt_finalize(const __grid_constant__ Par p, Scal* sc, int mode) { dt_finalize(p, sc, mode); }
+
+// the cells' CFL lengths, fixed with the grid: one plane for CalcDT to read instead of three
+__global__ void k_min_length(long long E, const double* di, const double* dj, const double* dk, double* dl) {
+    const long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (l >= E) return;
+    double m = di[l];
+    if (dj[l] < m) m = dj[l];
+    if (dk[l] < m) m = dk[l];
+    dl[l] = m;
+}
+// The minimum over the dt domain. finalize >= 0: the last block to finish goes on to finalize the dt in that mode
+// (one launch less on the step's chain); -1 where a tiled run reduces the minimum over its tiles first.
+__global__ void k_calcdt(Lay L, const __grid_constant__ Par p, GridP g, StateP s, Scal* sc, int finalize) {
     const Reg r = reg_dt(L, p);
     int i, j, k;
     double dtijk = HUGEV * 2.0;
@@ -446,10 +499,7 @@ __global__ void k_calcdt(Lay L, Par p, GridP g, StateP s, Scal* sc) {
             if (p.doBoris) Valf = p.Ca * Valf * rsq(p.Ca * p.Ca + Valf * Valf);
         }
         double vCFL = MagV + sqrt(sq(Cs) + sq(Valf)) + 0.0;
-        double dl = g.di[c];
-        if (g.dj[c] < dl) dl = g.dj[c];
-        if (g.dk[c] < dl) dl = g.dk[c];
-        dtijk = p.CFL * dl / vCFL;
+        dtijk = p.CFL * g.dl[c] / vCFL;
         if (dtijk != dtijk) { isnan_ = true; dtijk = HUGEV * 2.0; }
     }
     // bit patterns of non-negative doubles order like the values
@@ -477,43 +527,16 @@ __global__ void k_calcdt(Lay L, Par p, GridP g, StateP s, Scal* sc) {
         if (lane == 0) {
             atomicMin(&sc->dtMinBits, bits);
             if (nn) atomicAdd(&sc->nanCount, nn);
+            if (finalize >= 0) {
+                __threadfence();
+                if (atomicAdd(&sc->blocksDone, 1u) + 1u == gridDim.x * gridDim.y) {
+                    __threadfence();
+                    sc->blocksDone = 0u;
+                    dt_finalize(p, sc, finalize);
+                }
+            }
         }
     }
-}
-
-// UpdateStateData time bookkeeping (gamapp.F90:113-114, mhdgroup.F90:104-105) and the rest of CalcDT
-// (step.F90:103-166): checks, the tFin clamp and the 10*dt0 clamp. mode 1 = initial dt (Hatch).
-__global__ void k_dt_finalize(Par p, Scal* sc, int mode) {
-    if (mode == 0) {
-        sc->otime = sc->time;
-        sc->time = sc->time + sc->dt;
-        sc->ts = sc->ts + 1;
-        sc->t = sc->t + sc->dt;
-        if (sc->bGiven > 0) sc->bGiven--;
-    }
-    if (p.fixedTimestep) { sc->status = 0; return; }
-    double dtOld = sc->dt;
-    double dtMin = __longlong_as_double((long long)sc->dtMinBits);
-    if (sc->dtMinBits >= 0x7FF0000000000000ull || dtMin > HUGEV) dtMin = HUGEV;
-    int st = 0;
-    if (dtMin == HUGEV) st |= 1;
-    if (sc->ts > 0) {
-        if (dtOld / dtMin >= 10) st |= 2;
-        if ((sc->dt0 > TINY) && (dtMin / sc->dt0 <= p.limDT0)) st |= 2;
-        if (dtMin <= TINY) st |= 1;
-    }
-    if (sc->nanCount) st |= 4;
-    if (sc->waitFail) st |= 8;
-    double r = dtMin;
-    if ((sc->t + r) > p.tFin) r = dmax(p.tFin - sc->t, TINY);
-    if (sc->dt0 > TINY && r > 10.0 * sc->dt0) r = 10.0 * sc->dt0;
-    sc->dt = r;
-    sc->status = st;
-    sc->sticky |= st;
-    sc->lastNan = sc->nanCount;
-    sc->dtMinBits = 0x7FF0000000000000ull;
-    sc->nanCount = 0u;
-    sc->waitFail = 0u;   // reported in this step's status (and the sticky OR); the next step starts clear
 }
 
 // ================================================================================ boundary conditions
@@ -767,7 +790,7 @@ GridP Handle::gridP() const {
     g.volume = volume;
     for (int x = 0; x < 3; ++x) g.xyzcc[x] = xyzcc[x];
     for (int d = 0; d < 3; ++d) for (int x = 0; x < 3; ++x) g.xfc[d][x] = xfc[d][x];
-    g.di = di; g.dj = dj; g.dk = dk;
+    g.dl = dl;
     for (int d = 0; d < 3; ++d) {
         g.face[d] = face[d]; g.edge[d] = edge[d];
         for (int q = 0; q < 9; ++q) { g.Tf[d][q] = Tf[d][q]; g.Te[d][q] = Te[d][q]; }
@@ -795,6 +818,11 @@ void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st) {
     if (o) { k_b_check<<<grid, TPB, 0, st>>>(h.L, h.p, h.gridP(), h.S[h.cur ^ 1], 1, h.dScal); h.launches++; }
 }
 
+void launch_min_length(Handle& h, cudaStream_t st) {
+    k_min_length<<<nblk(h.L.E, 256), 256, 0, st>>>(h.L.E, h.di, h.dj, h.dk, h.dl);
+    h.launches++;
+}
+
 void launch_half_con(Handle& h, cudaStream_t st) {
     PrimP Wh;
     for (int v = 0; v < 5; ++v) Wh.w[v] = h.Wh[v];
@@ -818,11 +846,20 @@ void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB) {
     h.launches += 3;
 }
 
-void launch_calcdt_partial(Handle& h, const StateP& s, cudaStream_t st) {
-    const Lay& L = h.L;
-    k_calcdt<<<grid_plane(reg_dt(L, h.p), 256), 256, 0, st>>>(L, h.p, h.gridP(), s, h.dScal);
-    h.launches++;
+// CalcDT's own finalization saves a launch; the many blocks of a large grid pay more for counting one another (256^3:
+// 287 us against 268 and the launch's 4)
+static bool dt_in_one(const Handle& h) {
+    const dim3 g = grid_plane(reg_dt(h.L, h.p), 256);
+    return g.x * g.y <= 8192u;
 }
+static void launch_calcdt_mode(Handle& h, const StateP& s, int finalize, cudaStream_t st) {
+    const Lay& L = h.L;
+    const bool one = dt_in_one(h);
+    k_calcdt<<<grid_plane(reg_dt(L, h.p), 256), 256, 0, st>>>(L, h.p, h.gridP(), s, h.dScal, one ? finalize : -1);
+    h.launches++;
+    if (finalize >= 0 && !one) launch_dt_finalize(h, finalize, st);
+}
+void launch_calcdt_partial(Handle& h, const StateP& s, cudaStream_t st) { launch_calcdt_mode(h, s, -1, st); }
 
 void launch_dt_finalize(Handle& h, int mode, cudaStream_t st) {
     k_dt_finalize<<<1, 1, 0, st>>>(h.p, h.dScal, mode);
@@ -830,8 +867,7 @@ void launch_dt_finalize(Handle& h, int mode, cudaStream_t st) {
 }
 
 void launch_calcdt(Handle& h, const StateP& s, int mode, cudaStream_t st) {
-    launch_calcdt_partial(h, s, st);
-    launch_dt_finalize(h, mode, st);
+    launch_calcdt_mode(h, s, mode, st);
 }
 
 __global__ void k_to_f32(const double* src, float* dst, long long n) {
@@ -905,11 +941,11 @@ int ensure_f32(Handle& h) {
 }
 
 int kernels_per_step(const Handle& h) {
-    int n = 1 + 1;                      // begin, predict cells
+    int n = 1;                          // predict cells
     if (h.p.doMHD) n += 1 + 1 + 3;      // predict faces, Mom2Face (all directions), 3 edge kernels
     n += (h.p.do25D ? 2 : 3) + ((h.fuseUpdate && !h.closure) ? 0 : 1);   // fluxes + flux2deltas
     n += 1 + 1 + 1;                     // e2flux/copy, bflux2fld, update gas
-    n += 2 + 3 + 1;                     // calcdt + finalize, 3 BC kernels, final bflux2fld
+    n += (dt_in_one(h) ? 1 : 2) + 3 + 1;   // calcdt (+ finalize), 3 BC kernels, final bflux2fld
     n += ring_kernels_per_step(h);
     n += msph_kernels_per_step(h);
     if (h.closure) n += closure_kernels_per_step(h) + 1;   // + the conditional Flux2Deltas
@@ -921,6 +957,8 @@ int kernels_per_step(const Handle& h) {
 // names as the reference's printClocks tree (Advance > Gamera > Predictor, E-Field, Fluxes, ...).
 static const char* const kPhaseRange[NPHASE] = {"Predictor", "E-Field", "Fluxes", "Flux2Deltas", "Update", "DT",
                                                 "BCs"};   // BCs is pushed by step_enqueue_bcs
+
+constexpr long long BRANCH_CELLS = 100000;
 
 int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     cudaStream_t st = h.stream;
@@ -940,10 +978,18 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     const Par& p = h.p;
     GridP g = h.gridP();
     StateP nS = h.S[cur], oS = h.S[cur ^ 1];
+    // The fluxes and the E field, and the two predictors, run beside one another where they are far from filling the GPU:
+    // a step is a chain of dependent launches, and a small problem's step costs the length of that chain. Not in larger
+    // problems, which gain nothing and pay for the joins, and not where other problems' steps run beside this one.
+    // 4,096 cells 64 -> 39 us per step, 65,536 cells 144 -> 139 (212 -> 210 in 2.5D); with branches everywhere 1.2 M
+    // cells 1281 -> 1288, 256^3 +3% and a 24-member ensemble 2.23 -> 2.31 ms.
+    Branches br{h, st, ev == nullptr && h.alone && (long long)L.Nip * L.Njp * L.Nkp <= BRANCH_CELLS};
+    const float* corr = nullptr;
     const Reg cells = {0, L.Ni, 0, L.Nj, 0, L.Nk}, act = {L.is(), L.Nip, L.js(), L.Njp, L.ks(), L.Nkp};
     if (part != STEP_POST) {
     mark(PH_PREDICT);
-    k_step_begin<<<1, 1, 0, st>>>(h.dScal);
+    // learned closure: face corrections from the net on State n, needed by Flux2Deltas
+    if (h.closure && part == STEP_ALL) corr = closure_enqueue_corr(h, nS, br.go(SIDE_NET));
     if (p.doMHD) {
         Vec3P mf = {{nS.mf[0], nS.mf[1], nS.mf[2]}}, omf = {{oS.mf[0], oS.mf[1], oS.mf[2]}},
               hmf = {{h.H.mf[0], h.H.mf[1], h.H.mf[2]}}, hbA = {{h.hbA[0], h.hbA[1], h.hbA[2]}},
@@ -951,7 +997,7 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
         F32FaceOut fo{};
         if (h.prec == PREC_FP32FLUX)
             for (int x = 0; x < 3; ++x) { fo.hbA[x] = h.f32.hbA[x]; fo.nbA[x] = h.f32.nbA[x]; }
-        k_predict_faces<<<nblk(L.E / 2, 256), 256, 0, st>>>(L.E, p, g, mf, omf, hmf, hbA, nbA, fo, h.dScal);
+        k_predict_faces<<<nblk(L.E / 2, 256), 256, 0, br.go(SIDE_FLUX)>>>(L.E, p, g, mf, omf, hmf, hbA, nbA, fo, h.dScal);
         h.launches++;
     }
     PrimP Wh, Wn;
@@ -962,19 +1008,29 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
         for (int x = 0; x < 3; ++x) { fc.hb[x] = h.f32.hb[x]; fc.nb[x] = h.f32.nb[x]; }
     }
     k_predict_cells<<<grid_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, TPB), TPB, 0, st>>>(L, p, g, nS, oS, h.H, Wh, Wn, fc, h.dScal);
-    h.launches += 2;
+    h.launches += 1;
     if (p.doRing) launch_ring_bfix(h, h.H, st, h.prec == PREC_FP32FLUX);   // bFlux2Fld's ring fix
     if (p.predFixLFM) launch_predfix_lfm(h, h.H, st, h.prec == PREC_FP32FLUX);   // HackPredictor
+    if (p.doMHD) br.join(SIDE_FLUX);
     mark(PH_EFIELD);
+    // the flux kernels beside the E field's (after it where everything is on one stream)
+    cudaStream_t fs[3] = {st, st, st};
+    if (br.on && part == STEP_ALL) {
+        for (int d = 0; d < 3; ++d) fs[d] = br.go(SIDE_FLUX + d);
+        enqueue_fluxes(h, nS, fs);
+    }
     if (p.doMHD) {
-        enqueue_efield(h, nS, st);
+        enqueue_efield(h, nS, br);
         if (p.msph.on) launch_msph_efix(h, nS, st);   // HackE (mhdgroup.F90:40-44)
     }
+    if (br.on && part == STEP_ALL)
+        for (int d = 0; d < 3; ++d) br.join(SIDE_FLUX + d);
     }
     if (part == STEP_PRE) return (int)cudaGetLastError();
-    if (part == STEP_ALL) {
+    if (part == STEP_ALL && !br.on) {
+        const cudaStream_t fs[3] = {st, st, st};
         mark(PH_FLUXES);
-        enqueue_fluxes(h, nS, st);
+        enqueue_fluxes(h, nS, fs);
     }
     if (p.doRing) launch_ring_flux(h, st);   // stress.F90:134-139
     if (p.msph.on) launch_ion_flux(h, st);    // HackFlux (stress.F90:141-143)
@@ -990,9 +1046,10 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     }
     // without a closure the update computes the deltas itself (no dGasH/dGasM round trip through HBM)
     const bool fuse = h.fuseUpdate && !h.closure;
-    // learned closure: face corrections from the net on State n; a corrected update that fails positivity
-    // falls back to the plain fluxes (the second, conditional Flux2Deltas)
-    const float* corr = h.closure ? closure_enqueue_corr(h, nS, st) : nullptr;
+    // learned closure: a corrected update that fails positivity falls back to the plain fluxes (the second, conditional
+    // Flux2Deltas). With the ensembles' tile queue the net runs here.
+    if (h.closure && !corr) corr = closure_enqueue_corr(h, nS, st);
+    else if (corr) br.join(SIDE_NET);
     for (int pass = 0; pass < (fuse ? 0 : (corr ? 2 : 1)); ++pass) {
         const float* cq = pass == 0 ? corr : nullptr;
         const Scal* cond = pass == 0 ? nullptr : h.dScal;
@@ -1004,8 +1061,20 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
         if (pass == 1) h.launches++;
     }
     mark(PH_UPDATE);
-    // applyUpdate into the oState buffer (which becomes State n+1)
+    // applyUpdate into the oState buffer (which becomes State n+1); only the Boris update needs the new field
     Vec3P E = {{h.E[0], h.E[1], h.E[2]}};
+    const bool apart = !p.doBoris;
+    auto update = [&](cudaStream_t us) {
+        const dim3 gc = grid_plane(cells, TPB);
+        if (h.prec == PREC_FP32FLUX) {
+            if (fuse) k_update_gas<float, true><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], h.dScal);
+            else k_update_gas<float, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], h.dScal);
+        } else {
+            if (fuse) k_update_gas<double, true><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
+            else k_update_gas<double, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
+        }
+    };
+    if (apart) update(br.go(SIDE_FLUX));
     if (p.doRing && p.doMHD) launch_pole_e(h, h.E, st);   // mhdgroup.F90:139-142
     if (h.closure && p.doMHD) closure_enqueue_emf(h, st);
     k_e2flux<<<grid_plane(Reg{0, L.Ni + 1, 0, L.Nj + 1, 0, L.Nk + 1}, TPB), TPB, 0, st>>>(L, p, E, nS, oS, h.dScal);
@@ -1013,22 +1082,17 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     // which recomputes every cell before anything reads a ghost B
     if (p.doMHD) k_bflux2fld<<<grid_plane(cells, TPB), TPB, 0, st>>>(L, g, oS);
     else k_copy_b<<<nblk(L.E, 256), 256, 0, st>>>(L, nS, oS);
-    if (h.prec == PREC_FP32FLUX) {
-        if (fuse) k_update_gas<float, true><<<grid_plane(cells, TPB), TPB, 0, st>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], h.dScal);
-        else k_update_gas<float, false><<<grid_plane(cells, TPB), TPB, 0, st>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], h.dScal);
-    } else {
-        if (fuse) k_update_gas<double, true><<<grid_plane(cells, TPB), TPB, 0, st>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
-        else k_update_gas<double, false><<<grid_plane(cells, TPB), TPB, 0, st>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
-    }
-    h.launches += 4;
+    if (!apart) update(st);
+    else br.join(SIDE_FLUX);
+    h.launches += 3;
     if (p.msph.on) launch_apply_grav(h, oS, nS, st);   // mhdgroup.F90:60-65 (oS holds the new state)
     if (p.doRing) launch_ring_average(h, oS, st);   // mhdgroup.F90:68-74
     if (p.msph.on) launch_msph_perstep(h, oS, st);   // HackStep (gamapp.F90:104-109)
     // CalcDT (the per-cell minimum; finalized below, or after the tiles' minimum for a tiled run)
     mark(PH_DT);
-    launch_calcdt_partial(h, oS, st);
+    launch_calcdt_mode(h, oS, split ? -1 : 0, st);
     if (!split) {
-        step_enqueue_bcs(h, cur, ev);
+        step_enqueue_bcs(h, cur, ev, true);
         step_enqueue_ghosts(h, cur);
         mark(NPHASE);
     }
@@ -1036,9 +1100,9 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
 }
 
 // The rest of CalcDT, then EnforceBCs on the new state S[cur ^ 1]
-void step_enqueue_bcs(Handle& h, int cur, cudaEvent_t* ev) {
+void step_enqueue_bcs(Handle& h, int cur, cudaEvent_t* ev, bool finalized) {
     cudaStream_t st = h.stream;
-    launch_dt_finalize(h, 0, st);
+    if (!finalized) launch_dt_finalize(h, 0, st);
     if (ev) cudaEventRecord(ev[PH_BCS], st);
     nvtxRangePushA("BCs");
     launch_bcs(h, h.S[cur ^ 1], st, false);   // step_enqueue_ghosts rewrites every ghost B

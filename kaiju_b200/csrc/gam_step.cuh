@@ -37,6 +37,12 @@ struct Handle {
     int device = 0;
     cudaStream_t stream = nullptr;
     bool ownStream = false;
+    // streams for the kernels of a step that do not depend on one another (Branches, below); joined into `stream`
+    // before a step ends, so a caller sees one stream
+    static constexpr int NSIDE = 6;
+    bool alone = true;       // no other problem's step is enqueued beside this one's (ensembles, tiles on one GPU)
+    cudaStream_t side[NSIDE] = {};
+    cudaEvent_t forkEv = nullptr, joinEv[NSIDE] = {};
     int prec = PREC_FP64;
 
     // one pool holds every plane; planes are E doubles each
@@ -57,7 +63,7 @@ struct Handle {
     double* gflx[3][5];   // interface gas fluxes per direction (area-scaled)
     double* mflx[3][3];   // interface magnetic stresses per direction
     // grid metrics (owned)
-    double* volume; double* xyzcc[3]; double* xfc[3][3]; double* di; double* dj; double* dk;
+    double* volume; double* xyzcc[3]; double* xfc[3][3]; double* di; double* dj; double* dk; double* dl;
     double* face[3]; double* edge[3]; double* Tf[3][9]; double* Te[3][9]; double* Teb[3][4];
     double* xyz[3];       // corners (only kept when the grid was built on the device)
     // background field planes (own allocation, only with Model%doBackground), Grid_T layout per plane
@@ -91,6 +97,26 @@ struct Handle {
     StateP old_state() const { return S[cur ^ 1]; }
 };
 
+// Kernels beside the step's stream. go(q) returns side stream q, ordered after everything on st so far; join(q) makes
+// st wait for it. Off (a phase-timed step), every kernel stays on st.
+struct Branches {
+    Handle& h;
+    cudaStream_t st;
+    bool on;
+    cudaStream_t go(int q) {
+        if (!on) return st;
+        cudaEventRecord(h.forkEv, st);
+        cudaStreamWaitEvent(h.side[q], h.forkEv, 0);
+        return h.side[q];
+    }
+    void join(int q) {
+        if (!on) return;
+        cudaEventRecord(h.joinEv[q], h.side[q]);
+        cudaStreamWaitEvent(st, h.joinEv[q], 0);
+    }
+};
+enum { SIDE_FLUX = 0, SIDE_EDGE = 3, SIDE_NET = 5 };   // three flux directions, two edge directions, the closure's net
+
 // Enqueue one full stepGamera on h.stream with State n = S[cur]. Does not flip cur.
 // part: the whole step, or the part before the fluxes (predictor, E field) / after them (Flux2Deltas on),
 // for the ensembles' tile-queue flux kernel that runs between the two for all members at once
@@ -98,13 +124,15 @@ enum { STEP_ALL = 0, STEP_PRE = 1, STEP_POST = 2 };
 int step_enqueue(Handle& h, int cur, cudaEvent_t* phaseEv = nullptr, bool split = false, int part = STEP_ALL);
 // split = true stops after the per-cell CalcDT minimum (into Scal::dtMinBits); a tiled run then reduces
 // the minimum over its tiles and continues with step_enqueue_bcs, the halo fill and step_enqueue_ghosts
-void step_enqueue_bcs(Handle& h, int cur, cudaEvent_t* phaseEv = nullptr);
+// finalized: CalcDT's last block has already finalized the dt
+void step_enqueue_bcs(Handle& h, int cur, cudaEvent_t* phaseEv = nullptr, bool finalized = false);
 void step_enqueue_ghosts(Handle& h, int cur);
 void launch_calcdt_partial(Handle& h, const StateP& s, cudaStream_t st);
-void launch_dt_finalize(Handle& h, int mode, cudaStream_t st);
+void launch_dt_finalize(Handle& h, int mode, cudaStream_t st);   // after launch_calcdt_partial
 // phases recorded by step_enqueue when phaseEv is given (NPHASE+1 events)
 enum { PH_PREDICT = 0, PH_EFIELD, PH_FLUXES, PH_DELTAS, PH_UPDATE, PH_DT, PH_BCS, NPHASE };
 // Kernels used outside the step
+void launch_min_length(Handle& h, cudaStream_t st);   // Grid%di, dj, dk -> dl, after either changes
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st);
 // Scal::bGiven after State n and/or oState came from outside the step: set to its most, or found by checking the
 // states named (the other is known to be bFlux2Fld of its fluxes)
@@ -126,12 +154,13 @@ void closure_enqueue_emf(Handle& h, cudaStream_t st);
 int closure_kernels_per_step(const Handle& h);
 int closure_attach(Handle& h, ::gam_closure* c);   // shape check, geometry and periodicity from h
 // interface fluxes of all directions (gam_flux.cu)
-void enqueue_fluxes(Handle& h, const StateP& nS, cudaStream_t st);
+// st[d]: the stream of direction d
+void enqueue_fluxes(Handle& h, const StateP& nS, const cudaStream_t* st);
 void flux_kernels_init();
-void enqueue_fluxes_f32(Handle& h, const StateP& nS, cudaStream_t st);   // gam_flux_f32.cu
+void enqueue_fluxes_f32(Handle& h, const StateP& nS, const cudaStream_t* st);   // gam_flux_f32.cu
 void flux_kernels_init_f32();
 // E field of all edge directions (gam_efield.cu): Mom2Face + tiled EMF
-void enqueue_efield(Handle& h, const StateP& nS, cudaStream_t st);
+void enqueue_efield(Handle& h, const StateP& nS, Branches& br);
 void efield_kernels_init();
 void efield_kernels_init_f32();   // gam_efield_f32.cu
 // ring averaging about the LFM axis (gam_ring.cu)

@@ -224,7 +224,12 @@ void fan(gam_tiles* T, F f) {
 // one tiled step, every tile at parity cur ^ flip
 int enqueue_tiled_step(gam_tiles* T, int flip) {
     int rc = 0;
-    fan(T, [&](int q) { Handle& h = H(T, q); if (step_enqueue(h, h.cur ^ flip, nullptr, true) != 0) rc = GAM_ERR_CUDA; });
+    fan(T, [&](int q) {
+        Handle& h = H(T, q);
+        h.alone = !T->oneDevice;
+        if (step_enqueue(h, h.cur ^ flip, nullptr, true) != 0) rc = GAM_ERR_CUDA;
+        h.alone = true;
+    });
     k_tiles_dtmin<<<1, 32, 0, T->root>>>(T->dScals, (int)T->t.size());
     fan(T, [&](int q) { Handle& h = H(T, q); step_enqueue_bcs(h, h.cur ^ flip); });
     // the new states are at parity cur ^ flip ^ 1; Bxyz of the halo is recomputed, so it is not copied
@@ -291,11 +296,11 @@ int tiles_collect(gam_tiles* T) {
     return worst;
 }
 
-// kernels of one tiled step per tile: those of an ordinary step plus the halo fill (and the tiles'
+// kernels of one tiled step per tile: those of an ordinary step, the finalized dt and the halo fill (and the tiles'
 // dt minimum, counted on tile 0)
 void count_launches(gam_tiles* T) {
     T->launchesPerStep.assign(T->t.size(), 0);
-    for (size_t q = 0; q < T->t.size(); ++q) T->launchesPerStep[q] = kernels_per_step(H(T, (int)q)) + 1 + (q == 0);
+    for (size_t q = 0; q < T->t.size(); ++q) T->launchesPerStep[q] = kernels_per_step(H(T, (int)q)) + 2 + (q == 0);
 }
 
 }  // namespace
