@@ -199,11 +199,6 @@ int alloc_handle(gam_gpu* G, const gam_model_c* m) {
     ring_kernels_init();
     CK(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     h.ownStream = true;
-    for (int q = 0; q < Handle::NSIDE; ++q) {
-        CK(cudaStreamCreateWithFlags(&h.side[q], cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&h.joinEv[q], cudaEventDisableTiming));
-    }
-    CK(cudaEventCreateWithFlags(&h.forkEv, cudaEventDisableTiming));
     const size_t planes = 11 * 3 + 10 + 11 + 9 + 24 + 92 + 6;   // + the I and J edges' face velocities
     h.poolPlanes = planes;
     CK(cudaMalloc(&h.pool, sizeof(double) * L.E * planes));
@@ -853,11 +848,6 @@ void gam_gpu_destroy(gam_gpu_t* G) {
     if (G->copyStream) cudaStreamDestroy(G->copyStream);
     if (h.dScal) cudaFree(h.dScal);
     if (h.hScal) cudaFreeHost(h.hScal);
-    for (int q = 0; q < Handle::NSIDE; ++q) {
-        if (h.side[q]) cudaStreamDestroy(h.side[q]);
-        if (h.joinEv[q]) cudaEventDestroy(h.joinEv[q]);
-    }
-    if (h.forkEv) cudaEventDestroy(h.forkEv);
     if (h.stream && h.ownStream) cudaStreamDestroy(h.stream);
     if (h.msphpool) cudaFree(h.msphpool);
     delete G;

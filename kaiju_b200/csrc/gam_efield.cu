@@ -204,14 +204,15 @@ void enqueue_efield(Handle& h, const StateP& nS, Branches& br) {
         launch_mom2face<double>(L, g.volume, h.Wh[1], h.Wh[2], h.Wh[3], o, rv[2], rv[0], rv[1], st);
     }
     h.launches++;
-    for (int eD = 2; eD >= 0; --eD) {   // the last on st itself
-        const cudaStream_t es = eD > 0 ? br.go(SIDE_EDGE + eD - 1) : st;
+    for (int eD = 2; eD >= 0; --eD) {   // the last on the main branch
+        if (eD > 0) br.go(SIDE_EDGE + eD - 1);
         for (int x = 0; x < 3; ++x) {
             in32.Vf[x] = eD < 2 ? h.f32.VfE[eD][x] : h.f32.Vf[x];
             in64.Vf[x] = eD < 2 ? h.VfE[eD][x] : h.Vf[x];
         }
-        if (f32) launch_edge_dir_f32(h, in32, eD, re[eD], es);
-        else launch_edge_dir<double, double>(h, in64, eD, re[eD], es);
+        if (f32) launch_edge_dir_f32(h, in32, eD, re[eD], st);
+        else launch_edge_dir<double, double>(h, in64, eD, re[eD], st);
+        if (eD > 0) br.back();
     }
     br.join(SIDE_EDGE);
     br.join(SIDE_EDGE + 1);

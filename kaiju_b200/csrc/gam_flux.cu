@@ -40,12 +40,12 @@ void launch_flux_queue64(const FluxJob<double>* jobs, int njobs, long long ntile
     k_flux_queue<double, double><<<grid, 256, flux_queue_smem<double>(), st>>>(jobs, njobs, ntiles, counter);
 }
 
-void enqueue_fluxes(Handle& h, const StateP& nS, const cudaStream_t* st) {
+void enqueue_fluxes(Handle& h, const StateP& nS, Branches& br) {
     if (h.prec == PREC_FP32FLUX) {
-        enqueue_fluxes_f32(h, nS, st);
+        enqueue_fluxes_f32(h, nS, br);
         return;
     }
-    fluxes_all<double, double>(h, flux_src64(h, nS), st);
+    fluxes_all<double, double>(h, flux_src64(h, nS), br);
 }
 
 }  // namespace gam

@@ -30,9 +30,9 @@ static FluxSrc<float> flux_src32(Handle& h) {
     return in;
 }
 
-void enqueue_fluxes_f32(Handle& h, const StateP& nS, const cudaStream_t* st) {
+void enqueue_fluxes_f32(Handle& h, const StateP& nS, Branches& br) {
     (void)nS;
-    fluxes_all<float, float>(h, flux_src32(h), st);
+    fluxes_all<float, float>(h, flux_src32(h), br);
 }
 
 void flux_jobs32(Handle& h, std::vector<FluxJob<float>>& jobs, long long& first) {

@@ -504,13 +504,20 @@ static void flux_jobs_of(Handle& h, const FluxSrc<S>& in, const FluxOut<S> F[3],
 
 // CalcStress flux loop (stress.F90:84-128): I, J and (unless 2.5D) K interfaces
 template <typename T, typename S>
-static void fluxes_all(Handle& h, const FluxSrc<S>& in, const cudaStream_t* st) {
+static void fluxes_all(Handle& h, const FluxSrc<S>& in, Branches& br) {
     const Lay& L = h.L;
     int is = L.is(), ie = L.ie(), js = L.js(), je = L.je(), ks = L.ks(), ke = L.ke();
     if (h.p.do25D) ke = ks;
-    launch_flux_dir<T, S, 0>(h, in, mkreg(is, ie + 1, js, je, ks, ke), st[0]);
-    launch_flux_dir<T, S, 1>(h, in, mkreg(is, ie, js, je + 1, ks, ke), st[1]);
-    if (!h.p.do25D) launch_flux_dir<T, S, 2>(h, in, mkreg(is, ie, js, je, ks, ke + 1), st[2]);
+    br.go(SIDE_FLUX);
+    launch_flux_dir<T, S, 0>(h, in, mkreg(is, ie + 1, js, je, ks, ke), br.st);
+    br.back();
+    br.go(SIDE_FLUX + 1);
+    launch_flux_dir<T, S, 1>(h, in, mkreg(is, ie, js, je + 1, ks, ke), br.st);
+    br.back();
+    if (h.p.do25D) return;
+    br.go(SIDE_FLUX + 2);
+    launch_flux_dir<T, S, 2>(h, in, mkreg(is, ie, js, je, ks, ke + 1), br.st);
+    br.back();
 }
 
 }  // namespace gam

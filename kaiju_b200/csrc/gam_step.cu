@@ -983,13 +983,17 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     // problems, which gain nothing and pay for the joins, and not where other problems' steps run beside this one.
     // 4,096 cells 64 -> 39 us per step, 65,536 cells 144 -> 139 (212 -> 210 in 2.5D); with branches everywhere 1.2 M
     // cells 1281 -> 1288, 256^3 +3% and a 24-member ensemble 2.23 -> 2.31 ms.
-    Branches br{h, st, ev == nullptr && h.alone && (long long)L.Nip * L.Njp * L.Nkp <= BRANCH_CELLS};
+    Branches br(st, ev == nullptr && h.alone && (long long)L.Nip * L.Njp * L.Nkp <= BRANCH_CELLS);
     const float* corr = nullptr;
     const Reg cells = {0, L.Ni, 0, L.Nj, 0, L.Nk}, act = {L.is(), L.Nip, L.js(), L.Njp, L.ks(), L.Nkp};
     if (part != STEP_POST) {
     mark(PH_PREDICT);
     // learned closure: face corrections from the net on State n, needed by Flux2Deltas
-    if (h.closure && part == STEP_ALL) corr = closure_enqueue_corr(h, nS, br.go(SIDE_NET));
+    if (h.closure && part == STEP_ALL) {
+        br.go(SIDE_NET);
+        corr = closure_enqueue_corr(h, nS, st);
+        br.back();
+    }
     if (p.doMHD) {
         Vec3P mf = {{nS.mf[0], nS.mf[1], nS.mf[2]}}, omf = {{oS.mf[0], oS.mf[1], oS.mf[2]}},
               hmf = {{h.H.mf[0], h.H.mf[1], h.H.mf[2]}}, hbA = {{h.hbA[0], h.hbA[1], h.hbA[2]}},
@@ -997,7 +1001,9 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
         F32FaceOut fo{};
         if (h.prec == PREC_FP32FLUX)
             for (int x = 0; x < 3; ++x) { fo.hbA[x] = h.f32.hbA[x]; fo.nbA[x] = h.f32.nbA[x]; }
-        k_predict_faces<<<nblk(L.E / 2, 256), 256, 0, br.go(SIDE_FLUX)>>>(L.E, p, g, mf, omf, hmf, hbA, nbA, fo, h.dScal);
+        br.go(SIDE_FLUX);
+        k_predict_faces<<<nblk(L.E / 2, 256), 256, 0, st>>>(L.E, p, g, mf, omf, hmf, hbA, nbA, fo, h.dScal);
+        br.back();
         h.launches++;
     }
     PrimP Wh, Wn;
@@ -1014,23 +1020,18 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     if (p.doMHD) br.join(SIDE_FLUX);
     mark(PH_EFIELD);
     // the flux kernels beside the E field's (after it where everything is on one stream)
-    cudaStream_t fs[3] = {st, st, st};
-    if (br.on && part == STEP_ALL) {
-        for (int d = 0; d < 3; ++d) fs[d] = br.go(SIDE_FLUX + d);
-        enqueue_fluxes(h, nS, fs);
-    }
+    if (br.on && part == STEP_ALL) enqueue_fluxes(h, nS, br);
     if (p.doMHD) {
         enqueue_efield(h, nS, br);
         if (p.msph.on) launch_msph_efix(h, nS, st);   // HackE (mhdgroup.F90:40-44)
     }
     if (br.on && part == STEP_ALL)
-        for (int d = 0; d < 3; ++d) br.join(SIDE_FLUX + d);
+        for (int d = 0; d < (p.do25D ? 2 : 3); ++d) br.join(SIDE_FLUX + d);
     }
     if (part == STEP_PRE) return (int)cudaGetLastError();
     if (part == STEP_ALL && !br.on) {
-        const cudaStream_t fs[3] = {st, st, st};
         mark(PH_FLUXES);
-        enqueue_fluxes(h, nS, fs);
+        enqueue_fluxes(h, nS, br);
     }
     if (p.doRing) launch_ring_flux(h, st);   // stress.F90:134-139
     if (p.msph.on) launch_ion_flux(h, st);    // HackFlux (stress.F90:141-143)
@@ -1074,7 +1075,11 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
             else k_update_gas<double, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
         }
     };
-    if (apart) update(br.go(SIDE_FLUX));
+    if (apart) {
+        br.go(SIDE_FLUX);
+        update(st);
+        br.back();
+    }
     if (p.doRing && p.doMHD) launch_pole_e(h, h.E, st);   // mhdgroup.F90:139-142
     if (h.closure && p.doMHD) closure_enqueue_emf(h, st);
     k_e2flux<<<grid_plane(Reg{0, L.Ni + 1, 0, L.Nj + 1, 0, L.Nk + 1}, TPB), TPB, 0, st>>>(L, p, E, nS, oS, h.dScal);
@@ -1096,7 +1101,8 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
         step_enqueue_ghosts(h, cur);
         mark(NPHASE);
     }
-    return (int)cudaGetLastError();
+    const int rc = (int)cudaGetLastError();
+    return rc == 0 && br.failed ? -1 : rc;
 }
 
 // The rest of CalcDT, then EnforceBCs on the new state S[cur ^ 1]

@@ -1,6 +1,7 @@
 // Host-side handle of one GAMERA problem on one GPU and the step launcher.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <vector>
 #include "gam_common.cuh"
 
@@ -37,12 +38,7 @@ struct Handle {
     int device = 0;
     cudaStream_t stream = nullptr;
     bool ownStream = false;
-    // streams for the kernels of a step that do not depend on one another (Branches, below); joined into `stream`
-    // before a step ends, so a caller sees one stream
-    static constexpr int NSIDE = 6;
     bool alone = true;       // no other problem's step is enqueued beside this one's (ensembles, tiles on one GPU)
-    cudaStream_t side[NSIDE] = {};
-    cudaEvent_t forkEv = nullptr, joinEv[NSIDE] = {};
     int prec = PREC_FP64;
 
     // one pool holds every plane; planes are E doubles each
@@ -97,22 +93,51 @@ struct Handle {
     StateP old_state() const { return S[cur ^ 1]; }
 };
 
-// Kernels beside the step's stream. go(q) returns side stream q, ordered after everything on st so far; join(q) makes
-// st wait for it. Off (a phase-timed step), every kernel stays on st.
+// Kernels beside one another in a captured step: between go(q) and back(), launches on st go to side branch q of the graph,
+// which starts after everything on the main branch so far; join(q) makes the main branch wait for it. The branches are
+// dependency sets of the one captured stream (side streams with their events cost a problem 3 to 10 ms of set-up). Off,
+// every kernel follows the one before.
 struct Branches {
-    Handle& h;
+    static constexpr int NSIDE = 6;
+    using Nodes = std::vector<cudaGraphNode_t>;
     cudaStream_t st;
     bool on;
-    cudaStream_t go(int q) {
-        if (!on) return st;
-        cudaEventRecord(h.forkEv, st);
-        cudaStreamWaitEvent(h.side[q], h.forkEv, 0);
-        return h.side[q];
+    bool failed = false;   // a dependency call failed: the capture is not to be used
+    int cur = -1;
+    Nodes main, side[NSIDE];
+    Branches(cudaStream_t s, bool wanted) : st(s), on(wanted) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (on) on = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive;
+    }
+    void go(int q) {
+        if (!on) return;
+        main = deps();
+        cur = q;
+    }
+    void back() {
+        if (!on) return;
+        side[cur] = deps();
+        set(main);
     }
     void join(int q) {
         if (!on) return;
-        cudaEventRecord(h.joinEv[q], h.side[q]);
-        cudaStreamWaitEvent(st, h.joinEv[q], 0);
+        Nodes d = deps();
+        for (cudaGraphNode_t n : side[q])
+            if (std::find(d.begin(), d.end(), n) == d.end()) d.push_back(n);
+        set(d);
+    }
+
+private:
+    Nodes deps() {
+        cudaStreamCaptureStatus cs;
+        const cudaGraphNode_t* p = nullptr;
+        size_t n = 0;
+        if (cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &p, &n) != cudaSuccess) { failed = true; return Nodes(); }
+        return Nodes(p, p + n);
+    }
+    void set(Nodes& d) {
+        if (cudaStreamUpdateCaptureDependencies(st, d.data(), d.size(), cudaStreamSetCaptureDependencies) != cudaSuccess)
+            failed = true;
     }
 };
 enum { SIDE_FLUX = 0, SIDE_EDGE = 3, SIDE_NET = 5 };   // three flux directions, two edge directions, the closure's net
@@ -154,10 +179,10 @@ void closure_enqueue_emf(Handle& h, cudaStream_t st);
 int closure_kernels_per_step(const Handle& h);
 int closure_attach(Handle& h, ::gam_closure* c);   // shape check, geometry and periodicity from h
 // interface fluxes of all directions (gam_flux.cu)
-// st[d]: the stream of direction d
-void enqueue_fluxes(Handle& h, const StateP& nS, const cudaStream_t* st);
+// (every direction a branch of its own)
+void enqueue_fluxes(Handle& h, const StateP& nS, Branches& br);
 void flux_kernels_init();
-void enqueue_fluxes_f32(Handle& h, const StateP& nS, const cudaStream_t* st);   // gam_flux_f32.cu
+void enqueue_fluxes_f32(Handle& h, const StateP& nS, Branches& br);   // gam_flux_f32.cu
 void flux_kernels_init_f32();
 // E field of all edge directions (gam_efield.cu): Mom2Face + tiled EMF
 void enqueue_efield(Handle& h, const StateP& nS, Branches& br);
