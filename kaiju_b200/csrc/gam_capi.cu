@@ -729,7 +729,11 @@ int gam_gpu_fetch(gam_gpu_t* G, const char* name, double* out, long long n) {
         if (h.prec == PREC_FP64 && !h.p.doBoris) launch_half_con(h, h.stream);
         put(h.H.gas, 5);
     }
-    else if (s == "hmagflux") { put(h.H.mf, 3); e = fe; }
+    else if (s == "hmagflux") {
+        if (h.prec == PREC_FP64 && h.p.doMHD) launch_half_flux(h, h.stream);
+        put(h.H.mf, 3);
+        e = fe;
+    }
     else if (s == "hbxyz") put(h.H.b, 3);
     else if (s == "efld") put(h.E, 3);
     else if (s == "vf") put(h.Vf, 3);

@@ -19,7 +19,7 @@ static FluxSrc<double> flux_src64(Handle& h, const StateP& nS) {
     for (int d = 0; d < 3; ++d) {
         for (int q = 0; q < 9; ++q) in.Tf[d][q] = h.Tf[d][q];
         in.face[d] = h.face[d];
-        in.bn[d] = h.H.mf[d];
+        in.bn[d] = h.hbA[d];
         for (int x = 0; x < 3; ++x) in.fcB0[d][x] = h.fcB0[d][x];
         in.b0[d] = h.bFlux0[d];
     }

@@ -141,10 +141,7 @@ __device__ __forceinline__ void flux_tile_body(const Lay& L, const Par& p, const
             for (int m = 0; m < 4; ++m) nQ[m] = T(sLim[(5 + x) * LB + lo(m)]);
             recon(Q, nQ, BL[x], BR[x]);
         }
-        // FP64: the half-state flux over the area (stress.F90:301); FP32: the stored flux/area
-        T Bn;
-        if constexpr (std::is_same<S, double>::value) Bn = T(__ldg(&in.bn[D][c]) / faB);
-        else Bn = T(__ldg(&in.bn[D][c]));
+        const T Bn = T(__ldg(&in.bn[D][c]));   // the half-state flux over the area (stress.F90:301)
         T mF[3] = {T(0), T(0), T(0)};
         if constexpr (BG) {   // background field on the face (stress.F90:302-305)
             T B0[3];
@@ -313,10 +310,7 @@ k_flux_tile(Lay L, Par p, const __grid_constant__ FluxMaps maps, FluxSrc<S> in, 
             for (int m = 0; m < 4; ++m) nQ[m] = T(sLim[(5 + x) * LB + lo(m)]);
             recon(Q, nQ, BL[x], BR[x]);
         }
-        // FP64: the half-state flux over the area (stress.F90:301); FP32: the stored flux/area
-        T Bn;
-        if constexpr (std::is_same<S, double>::value) Bn = T(__ldg(&in.bn[D][c]) / faB);
-        else Bn = T(__ldg(&in.bn[D][c]));
+        const T Bn = T(__ldg(&in.bn[D][c]));   // the half-state flux over the area (stress.F90:301)
         T mF[3] = {T(0), T(0), T(0)};
         if constexpr (BG) {   // background field on the face (stress.F90:302-305)
             T B0[3];

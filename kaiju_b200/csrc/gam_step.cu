@@ -55,12 +55,13 @@ __global__ void k_predict_faces(long long E, Par p, GridP g, Vec3P mf, Vec3P omf
             double dQ = (Q[e] - oQ[e]) * iodt;
             H[e] = Q[e] + pdt * dQ;
             const double ia = 1.0 / dmax(A[e], TINY);
-            hb[e] = H[e] * ia;
+            // double precision: rounded once, as the fluxes take the face field from it
+            hb[e] = o.hbA[0] ? H[e] * ia : H[e] / dmax(A[e], TINY);
             nb[e] = (p.doLFMLim ? Q[e] : H[e]) * ia;
         }
-        // the half-state flux: bFlux2Fld of the half state reads it
-        *reinterpret_cast<double2*>(hmf.v[c] + l) = make_double2(H[0], H[1]);
         if (o.hbA[0]) {
+            // the half-state flux, for inspection (in double precision it is hbA times the area)
+            *reinterpret_cast<double2*>(hmf.v[c] + l) = make_double2(H[0], H[1]);
             *reinterpret_cast<float2*>(o.hbA[c] + l) = make_float2(float(hb[0]), float(hb[1]));
             *reinterpret_cast<float2*>(o.nbA[c] + l) = make_float2(float(nb[0]), float(nb[1]));
         } else {
@@ -164,6 +165,12 @@ __global__ void k_half_con(Lay L, Par p, PrimP Wh, StateP h) {
     for (int v = 0; v < 5; ++v) w[v] = Wh.w[v][c];
     cellP2C(p, w, U);
     for (int v = 0; v < 5; ++v) h.gas[v][c] = U[v];
+}
+// the half-state fluxes from the face fields (FP64, for inspection)
+__global__ void k_half_flux(long long E, GridP g, Vec3P hbA, Vec3P hmf) {
+    const long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (l >= E) return;
+    for (int d = 0; d < 3; ++d) hmf.v[d][l] = hbA.v[d][l] * dmax(g.face[d][l], TINY);
 }
 // Scal::bGiven after a state came from outside: `steps`, raised by k_b_check for a state whose Bxyz is not, bit for
 // bit, what a step leaves: bFlux2Fld of its fluxes, with the cells across the axis taking their conjugates'
@@ -827,6 +834,12 @@ void launch_half_con(Handle& h, cudaStream_t st) {
     PrimP Wh;
     for (int v = 0; v < 5; ++v) Wh.w[v] = h.Wh[v];
     k_half_con<<<grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB), TPB, 0, st>>>(h.L, h.p, Wh, h.H);
+    h.launches++;
+}
+
+void launch_half_flux(Handle& h, cudaStream_t st) {
+    k_half_flux<<<nblk(h.L.E, 256), 256, 0, st>>>(h.L.E, h.gridP(), Vec3P{{h.hbA[0], h.hbA[1], h.hbA[2]}},
+                                                  Vec3P{{h.H.mf[0], h.H.mf[1], h.H.mf[2]}});
     h.launches++;
 }
 

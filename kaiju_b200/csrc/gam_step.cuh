@@ -165,6 +165,8 @@ void mark_b_given(Handle& h, cudaStream_t st);
 void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st);
 // h.H.gas from the half-state primitives, which the FP64 step without Boris does not write
 void launch_half_con(Handle& h, cudaStream_t st);
+// h.H.mf from the face fields, which the FP64 step does not write
+void launch_half_flux(Handle& h, cudaStream_t st);
 // withB: ghost B copied with the gas (set-up); a step leaves it to the bFlux2Fld of the ghost cells that follows
 void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB = true);
 void launch_calcdt(Handle& h, const StateP& s, int mode, cudaStream_t st);   // mode 0: in-step, 1: initial (no time advance)
