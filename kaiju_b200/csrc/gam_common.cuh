@@ -243,11 +243,12 @@ __device__ __forceinline__ T central8(const T* q) {
 }
 
 // gamCellBxyz (gridutils.F90:648-680): second-order cell field from the six face fluxes
-__device__ __forceinline__ void cellBxyz(const Lay& L, const GridP& g, double* const* mf, long long c, double* B) {
+__device__ __forceinline__ void cellBxyz(const Lay& L, const GridP& g, const double* lo, const double* hi, long long c,
+                                         double* B) {   // from the lower and upper face fluxes
     double idV = 1.0 / g.volume[c];
-    double fI = mf[0][c], fJ = mf[1][c], fK = mf[2][c];
+    double fI = lo[0], fJ = lo[1], fK = lo[2];
     long long ci = c + 1, cj = c + L.P, ck = c + (long long)L.P * L.Q;
-    double fIp = mf[0][ci], fJp = mf[1][cj], fKp = mf[2][ck];
+    double fIp = hi[0], fJp = hi[1], fKp = hi[2];
     double Div = fIp - fI + fJp - fJ + fKp - fK;
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
@@ -255,6 +256,11 @@ __device__ __forceinline__ void cellBxyz(const Lay& L, const GridP& g, double* c
                     fJ * g.xfc[1][x][c] - fK * g.xfc[2][x][c]) * idV;
         B[x] = b - Div * g.xyzcc[x][c] * idV;
     }
+}
+__device__ __forceinline__ void cellBxyz(const Lay& L, const GridP& g, double* const* mf, long long c, double* B) {
+    const double lo[3] = {mf[0][c], mf[1][c], mf[2][c]};
+    const double hi[3] = {mf[0][c + 1], mf[1][c + L.P], mf[2][c + (long long)L.P * L.Q]};
+    cellBxyz(L, g, lo, hi, c, B);
 }
 
 }  // namespace gam

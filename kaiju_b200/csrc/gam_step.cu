@@ -247,8 +247,7 @@ __global__ void k_flux2deltas(Lay L, Par p, GridP g, FluxOut<O> FI, FluxOut<O> F
 // ================================================================================ update
 // E2Flux (fields.F90:18-51) on the active faces; every other face element carries State n over
 // (the reference updates State in place after copying it to oState).
-__global__ void k_e2flux(Lay L, Par p, Vec3P E, StateP nS, StateP oNew, const Scal* sc) {
-    Reg r = {0, L.Ni + 1, 0, L.Nj + 1, 0, L.Nk + 1};
+__global__ void k_e2flux(Lay L, Par p, Vec3P E, StateP nS, StateP oNew, Reg r, const Scal* sc) {
     int i, j, k;
     if (!reg_plane(r, i, j, k)) return;
     long long c = L.at(i, j, k);
@@ -269,8 +268,7 @@ __global__ void k_e2flux(Lay L, Par p, Vec3P E, StateP nS, StateP oNew, const Sc
     oNew.mf[0][c] = m0; oNew.mf[1][c] = m1; oNew.mf[2][c] = m2;
 }
 
-__global__ void k_bflux2fld(Lay L, GridP g, StateP s) {
-    Reg r = {0, L.Ni, 0, L.Nj, 0, L.Nk};
+__global__ void k_bflux2fld(Lay L, GridP g, StateP s, Reg r) {
     int i, j, k;
     if (!reg_plane(r, i, j, k)) return;
     long long c = L.at(i, j, k);
@@ -330,8 +328,7 @@ __device__ void cellBoris(const Par& p, double* U2, const double* U0, const doub
 // instead of read from the dGasH/dGasM planes
 template <typename O, bool FUSED>
 __global__ void k_update_gas(Lay L, Par p, GridP g, StateP nS, StateP oNew, PrimP dGH, Vec3P dGM, FluxOut<O> FI,
-                             FluxOut<O> FJ, FluxOut<O> FK, const Scal* sc) {
-    Reg r = {0, L.Ni, 0, L.Nj, 0, L.Nk};
+                             FluxOut<O> FJ, FluxOut<O> FK, Reg r, const Scal* sc) {
     int i, j, k;
     if (!reg_plane(r, i, j, k)) return;
     long long c = L.at(i, j, k);
@@ -745,6 +742,101 @@ __global__ void k_bc_k(Lay L, Par p, StateP s, int withB) {
     }
 }
 
+// All six sides periodic: EnforceBCs and the bFlux2Fld of the ghost cells in one launch. The three sweeps copy along one
+// axis each, so a ghost value is that of the active element its three indices map to one by one (images of other
+// images never arise, and what is read is never written); the field of a ghost cell comes from the fluxes its six faces
+// get. The update then need not carry over more than the layer CalcDT reads (6 planes instead of 12 for 4 cells across
+// k), and the faces that no sweep fills are carried over here, from the old state. Bound by the metrics and fluxes it
+// reads for the field, and on a small problem by its place in the step's chain of launches. The sweeps and the full
+// update against this, steps and their output together: 32x32x4 (10 steps) 668 -> 636 us, 128x128x4 (20) 3283 -> 3184,
+// 256x256x1 (20) 5298 -> 4942, 96x83x70 with FP32 fluxes (10) 4202 -> 4141. Joining the update's E2Flux and bFlux2Fld as
+// well was slower (256^3: 79 us a step) and is not done.
+struct PerMap {   // one axis: elements s..e of an extent n wrap; flat: 2.5D, where every layer takes the active one
+    int s, e, n, nG, flat;
+    __device__ __forceinline__ int wrap(int m) const { return n >= nG ? m : m % n; }   // m < nG: seldom a division
+    __device__ __forceinline__ int src(int x, bool normal) const {   // normal: faces across this axis
+        if (x < s) return flat ? s : e - wrap(s - x - 1);
+        if (flat) return x <= s + nG ? s : x;
+        const int up = normal ? 1 : 0, m = x - up - e;   // the m-th layer above
+        return m >= 1 && m <= nG ? s + up + wrap(m - 1) : x;
+    }
+};
+// what lies outside the active cells, one element more along each axis for the faces (2.5D: everything), i fastest;
+// 32-bit indices (the host checks)
+struct PerBox { int n[3], a0[3], na[3]; unsigned total; };
+__device__ __forceinline__ void per_ijk(const PerBox& b, unsigned t, int& i, int& j, int& k) {
+    const unsigned ni = b.n[0], sK = ni * b.n[1], nK = sK * (b.n[2] - b.na[2]);
+    if (t < nK) {
+        k = t / sK; t -= k * sK;
+        if (k >= b.a0[2]) k += b.na[2];
+        j = t / ni; i = t - j * ni;
+        return;
+    }
+    t -= nK;
+    const unsigned sJ = ni * b.na[2], nJ = sJ * (b.n[1] - b.na[1]);
+    if (t < nJ) {
+        j = t / sJ; t -= j * sJ;
+        if (j >= b.a0[1]) j += b.na[1];
+        k = t / ni; i = t - k * ni;
+        k += b.a0[2];
+        return;
+    }
+    t -= nJ;
+    const unsigned gi = ni - b.na[0], q = t / gi;
+    i = t - q * gi;
+    if (i >= b.a0[0]) i += b.na[0];
+    k = q / b.na[1]; j = q - k * b.na[1];
+    k += b.a0[2]; j += b.a0[1];
+}
+__global__ void k_bc_periodic(const __grid_constant__ Lay L, const __grid_constant__ GridP g, const __grid_constant__ StateP old,
+                              const __grid_constant__ StateP s,
+                              const __grid_constant__ PerBox box, const __grid_constant__ PerMap mi,
+                              const __grid_constant__ PerMap mj, const __grid_constant__ PerMap mk) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= box.total) return;
+    int i, j, k;
+    per_ijk(box, t, i, j, k);
+    // the D face's source and value; a face in the last layer across another axis belongs to no cell and carries over
+    auto face = [&](int d, int ii, int jj, int kk, long long& q, bool& last) {
+        const int si = mi.src(ii, d == 0), sj = mj.src(jj, d == 1), sk = mk.src(kk, d == 2);
+        last = si == L.Ni || sj == L.Nj || sk == L.Nk;
+        q = L.at(si, sj, sk);
+        return last ? old.mf[d][q] : s.mf[d][q];
+    };
+    const long long c = L.at(i, j, k);
+    const bool cell = i < L.Ni && j < L.Nj && k < L.Nk;
+    bool put[3];
+    double gas[5], lo[3], hi[3], B[3];
+    const long long cs = L.at(mi.src(i, false), mj.src(j, false), mk.src(k, false));
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        long long q;
+        bool last;
+        lo[d] = face(d, i, j, k, q, last);
+        put[d] = last || q != c;
+    }
+    if (cell) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) gas[v] = s.gas[v][cs];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            long long q;
+            bool last;
+            hi[d] = face(d, i + (d == 0), j + (d == 1), k + (d == 2), q, last);
+        }
+        cellBxyz(L, g, lo, hi, c, B);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) if (put[d]) s.mf[d][c] = lo[d];
+    if (!cell) return;
+    if (cs != c) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) s.gas[v][c] = gas[v];
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) s.b[x][c] = B[x];
+}
+
 // DivB (gridutils.F90:717-770) partial sums, one per block, reduced in a fixed order afterwards
 __global__ void k_divb_partial(Lay L, GridP g, int bg, StateP s, double* partial) {
     Reg r = {L.is(), L.Nip, L.js(), L.Njp, L.ks(), L.Nkp};
@@ -844,7 +936,8 @@ void launch_half_flux(Handle& h, cudaStream_t st) {
 }
 
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st) {
-    k_bflux2fld<<<grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB), TPB, 0, st>>>(h.L, h.gridP(), s);
+    const Reg r = {0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk};
+    k_bflux2fld<<<grid_plane(r, TPB), TPB, 0, st>>>(h.L, h.gridP(), s, r);
     h.launches++;
     if (h.p.doRing) launch_ring_bfix(h, s, st);   // gridutils.F90:298-300
 }
@@ -857,6 +950,27 @@ void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB) {
     k_bc_j<<<dim3(nblk((long long)(L.Ni + 1) * (L.Nk + 1), TPB), serialJ ? 1 : 2 * L.nG), TPB, 0, st>>>(L, h.p, s, withB, serialJ);
     k_bc_k<<<dim3(nblk((long long)(L.Ni + 1) * (L.Nj + 1), TPB), 2 * L.nG), TPB, 0, st>>>(L, h.p, s, withB);
     h.launches += 3;
+}
+
+static PerBox per_box(const Handle& h) {
+    const Lay& L = h.L;
+    PerBox b = {{L.Ni + 1, L.Nj + 1, L.Nk + 1}, {L.is(), L.js(), L.ks()}, {L.Nip, L.Njp, h.p.do25D ? 0 : L.Nkp}, 0u};
+    const long long n = (long long)b.n[0] * b.n[1] * b.n[2] - (long long)b.na[0] * b.na[1] * b.na[2];
+    b.total = n < (1ll << 31) ? (unsigned)n : 0u;
+    return b;
+}
+// the sides and the sizes that k_bc_periodic takes
+static bool bc_in_one(const Handle& h) {
+    for (int q = 0; q < 6; ++q) if (h.p.bc[q] != BC_PERIODIC) return false;
+    return !h.p.doRing && !h.p.msph.on && !(h.p.do25D && h.L.Nkp > 1) && per_box(h).total > 0u;
+}
+static void launch_bc_periodic(Handle& h, const StateP& n, const StateP& s, cudaStream_t st) {
+    const Lay& L = h.L;
+    const PerBox b = per_box(h);
+    const PerMap mi = {L.is(), L.ie(), L.Nip, L.nG, 0}, mj = {L.js(), L.je(), L.Njp, L.nG, 0},
+                 mk = {L.ks(), L.ke(), L.Nkp, L.nG, h.p.do25D};
+    k_bc_periodic<<<nblk(b.total, TPB), TPB, 0, st>>>(L, h.gridP(), n, s, b, mi, mj, mk);
+    h.launches++;
 }
 
 // CalcDT's own finalization saves a launch; the many blocks of a large grid pay more for counting one another (256^3:
@@ -953,12 +1067,12 @@ int ensure_f32(Handle& h) {
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
-int kernels_per_step(const Handle& h) {
+int kernels_per_step(const Handle& h, bool split) {
     int n = 1;                          // predict cells
     if (h.p.doMHD) n += 1 + 1 + 3;      // predict faces, Mom2Face (all directions), 3 edge kernels
     n += (h.p.do25D ? 2 : 3) + ((h.fuseUpdate && !h.closure) ? 0 : 1);   // fluxes + flux2deltas
     n += 1 + 1 + 1;                     // e2flux/copy, bflux2fld, update gas
-    n += (dt_in_one(h) ? 1 : 2) + 3 + 1;   // calcdt (+ finalize), 3 BC kernels, final bflux2fld
+    n += (!split && dt_in_one(h) ? 1 : 2) + (!split && bc_in_one(h) ? 1 : 3 + 1);   // calcdt (+ finalize), 3 BC kernels, final bflux2fld
     n += ring_kernels_per_step(h);
     n += msph_kernels_per_step(h);
     if (h.closure) n += closure_kernels_per_step(h) + 1;   // + the conditional Flux2Deltas
@@ -998,7 +1112,13 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     // cells 1281 -> 1288, 256^3 +3% and a 24-member ensemble 2.23 -> 2.31 ms.
     Branches br(st, ev == nullptr && h.alone && (long long)L.Nip * L.Njp * L.Nkp <= BRANCH_CELLS);
     const float* corr = nullptr;
-    const Reg cells = {0, L.Ni, 0, L.Nj, 0, L.Nk}, act = {L.is(), L.Nip, L.js(), L.Njp, L.ks(), L.Nkp};
+    // what the update writes: everything, or, where k_bc_periodic writes all that lies further out, the active cells and
+    // the layer around them that CalcDT reads
+    const bool one = !split && bc_in_one(h);
+    const Reg cells = one ? Reg{L.is() - 1, L.Nip + 2, L.js() - 1, L.Njp + 2, L.ks() - 1, L.Nkp + 2}
+                          : Reg{0, L.Ni, 0, L.Nj, 0, L.Nk};
+    const Reg faces = {cells.i0, cells.ni + 1, cells.j0, cells.nj + 1, cells.k0, cells.nk + 1};
+    const Reg act = {L.is(), L.Nip, L.js(), L.Njp, L.ks(), L.Nkp};
     if (part != STEP_POST) {
     mark(PH_PREDICT);
     // learned closure: face corrections from the net on State n, needed by Flux2Deltas
@@ -1081,11 +1201,11 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     auto update = [&](cudaStream_t us) {
         const dim3 gc = grid_plane(cells, TPB);
         if (h.prec == PREC_FP32FLUX) {
-            if (fuse) k_update_gas<float, true><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], h.dScal);
-            else k_update_gas<float, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], h.dScal);
+            if (fuse) k_update_gas<float, true><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], cells, h.dScal);
+            else k_update_gas<float, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F32[0], F32[1], F32[2], cells, h.dScal);
         } else {
-            if (fuse) k_update_gas<double, true><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
-            else k_update_gas<double, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], h.dScal);
+            if (fuse) k_update_gas<double, true><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], cells, h.dScal);
+            else k_update_gas<double, false><<<gc, TPB, 0, us>>>(L, p, g, nS, oS, dGH, dGM, F64[0], F64[1], F64[2], cells, h.dScal);
         }
     };
     if (apart) {
@@ -1095,10 +1215,10 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     }
     if (p.doRing && p.doMHD) launch_pole_e(h, h.E, st);   // mhdgroup.F90:139-142
     if (h.closure && p.doMHD) closure_enqueue_emf(h, st);
-    k_e2flux<<<grid_plane(Reg{0, L.Ni + 1, 0, L.Nj + 1, 0, L.Nk + 1}, TPB), TPB, 0, st>>>(L, p, E, nS, oS, h.dScal);
+    k_e2flux<<<grid_plane(faces, TPB), TPB, 0, st>>>(L, p, E, nS, oS, faces, h.dScal);
     // bFlux2Fld of the update; with ring averaging its ring fix is left to the RingAverage bFlux2Fld,
     // which recomputes every cell before anything reads a ghost B
-    if (p.doMHD) k_bflux2fld<<<grid_plane(cells, TPB), TPB, 0, st>>>(L, g, oS);
+    if (p.doMHD) k_bflux2fld<<<grid_plane(cells, TPB), TPB, 0, st>>>(L, g, oS, cells);
     else k_copy_b<<<nblk(L.E, 256), 256, 0, st>>>(L, nS, oS);
     if (!apart) update(st);
     else br.join(SIDE_FLUX);
@@ -1110,8 +1230,13 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     mark(PH_DT);
     launch_calcdt_mode(h, oS, split ? -1 : 0, st);
     if (!split) {
-        step_enqueue_bcs(h, cur, ev, true);
-        step_enqueue_ghosts(h, cur);
+        if (one) {
+            mark(PH_BCS);
+            launch_bc_periodic(h, nS, oS, st);
+        } else {
+            step_enqueue_bcs(h, cur, ev, true);
+            step_enqueue_ghosts(h, cur);
+        }
         mark(NPHASE);
     }
     const int rc = (int)cudaGetLastError();

@@ -171,7 +171,7 @@ void launch_half_flux(Handle& h, cudaStream_t st);
 void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB = true);
 void launch_calcdt(Handle& h, const StateP& s, int mode, cudaStream_t st);   // mode 0: in-step, 1: initial (no time advance)
 double launch_divb(Handle& h, double* scratchDev, cudaStream_t st);
-int kernels_per_step(const Handle& h);
+int kernels_per_step(const Handle& h, bool split = false);   // split: as a tile's step is taken
 // learned closure in the step (gam_closure.cu): the net on State n and its face corrections (24 float
 // planes, area-scaled) before Flux2Deltas; after it the positivity check that sets Scal::closureReject
 const float* closure_enqueue_corr(Handle& h, const StateP& nS, cudaStream_t st);

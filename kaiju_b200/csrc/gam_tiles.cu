@@ -296,11 +296,11 @@ int tiles_collect(gam_tiles* T) {
     return worst;
 }
 
-// kernels of one tiled step per tile: those of an ordinary step, the finalized dt and the halo fill (and the tiles'
+// kernels of one tiled step per tile: those of a step in its parts and the halo fill (and the tiles'
 // dt minimum, counted on tile 0)
 void count_launches(gam_tiles* T) {
     T->launchesPerStep.assign(T->t.size(), 0);
-    for (size_t q = 0; q < T->t.size(); ++q) T->launchesPerStep[q] = kernels_per_step(H(T, (int)q)) + 2 + (q == 0);
+    for (size_t q = 0; q < T->t.size(); ++q) T->launchesPerStep[q] = kernels_per_step(H(T, (int)q), true) + 1 + (q == 0);
 }
 
 }  // namespace

@@ -1,6 +1,6 @@
 """The step's kernels at the sizes where their launch rules change and where a tile, a run of faces or a ghost layer ends
 early. Against the oracle the bound is the parity tests' 1e-10; variants that differ only in the launch give the same
-bits."""
+bits. The periodic sides' index map is checked on the CPU too, against the three sweeps it stands for."""
 import numpy as np
 import pytest
 
@@ -8,6 +8,74 @@ from helpers import mirror_to_gpu, oracle_and_gpu, per_var_rel, resync
 
 TOL = 1e-10
 STATE = ("gas", "magflux", "bxyz")
+
+
+def _axis(n, normal, flat, ng=4):
+    """Where each element of an axis of n active cells is taken from: the map of k_bc_periodic"""
+    s, e = ng, ng + n - 1
+    src = np.arange(n + 2 * ng + 1)
+    for x in range(len(src)):
+        up = 1 if normal and not flat else 0
+        if x < s:
+            src[x] = s if flat else e - (s - x - 1) % n
+        elif flat:
+            src[x] = s if x <= s + ng else x
+        elif 1 <= x - up - e <= ng:
+            src[x] = s + up + (x - up - e - 1) % n
+    return src
+
+
+def _sweeps(a, n, comp, d25, ng=4):
+    """EnforceBCs of six periodic sides layer by layer (comp: 0-2 the faces across that axis, 3 the cells)"""
+    a = a.copy()
+    for d in range(3):
+        v, s, e = np.moveaxis(a, d, 0), ng, ng + n[d] - 1
+        flat, up = d == 2 and d25, 1 if comp == d else 0
+        for m in range(ng):
+            v[s - 1 - m] = v[s if flat else e - m % n[d]]
+            if flat:
+                v[s + 1 + m] = v[s]
+            else:
+                v[e + 1 + m + up] = v[s + m % n[d] + up]
+    return a
+
+
+@pytest.mark.parametrize("n,d25", [((8, 5, 6), False), ((8, 2, 3), False), ((16, 7, 1), True), ((8, 1, 1), True)])
+def test_periodic_map_equals_sweeps(n, d25):
+    for comp in range(4):
+        a = np.random.default_rng(comp).normal(size=tuple(q + 9 for q in n))
+        m = [_axis(n[d], comp == d, d == 2 and d25) for d in range(3)]
+        want, got = _sweeps(a, n, comp, d25), a[np.ix_(*m)]
+        if comp == 3:   # the cells end one element before the faces
+            want, got = want[:-1, :-1, :-1], got[:-1, :-1, :-1]
+        assert np.array_equal(want, got)
+        assert all(np.array_equal(q[q], q) for q in m)   # nothing that is read is written
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "fp32flux"])
+@pytest.mark.parametrize("n,kw", [((16, 5, 6), {}), ((16, 4, 4), dict(rmeth="7UP")), ((40, 9, 1), {}), ((32, 13, 1), dict(doMHD=False))])
+def test_periodic_sides(gpu_lib, oracle_lib, n, kw, prec):
+    """Steps with six periodic sides against the oracle, ghosts and the faces beyond them included, and the ghosts against
+    the sweeps exactly."""
+    from kaiju_b200 import gamera as gm
+    o, g = oracle_and_gpu("ot", n, **kw)
+    with g:
+        if prec == "fp32flux":
+            g.set_precision(gm.GAM_FP32FLUX)
+        for _ in range(2):
+            o.step()
+            g.step()
+            for name in STATE if prec == "fp64" else ():
+                assert max(per_var_rel(g.fetch(name), o.get(name))) <= TOL, name
+            for name in ("gas", "magflux"):
+                a = g.fetch(name)
+                for v in range(a.shape[3]):
+                    ng1 = np.pad(a[..., v], ((0, 1),) * 3) if name == "gas" else a[..., v]
+                    want = _sweeps(ng1, n, v if name == "magflux" else 3, n[2] == 1)
+                    cut = slice(None, -1) if name == "gas" else slice(None)
+                    assert np.array_equal(want[cut, cut, cut], a[..., v]), (name, v)
+            resync(o, g)
 
 
 @pytest.mark.gpu
