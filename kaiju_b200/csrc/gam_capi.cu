@@ -331,7 +331,7 @@ int launch_one_step(gam_gpu* G) {
     } else {
         if (step_enqueue(h, h.cur) != 0) return GAM_ERR_CUDA;
     }
-    h.cur ^= 1;
+    h.stepped();
     return GAM_OK;
 }
 
@@ -624,7 +624,7 @@ int gam_gpu_profile_phases(gam_gpu_t* G, int nsteps, double* ms, int nphase) {
     for (int q = 0; q < NPHASE; ++q) ms[q] = 0.0;
     for (int s = 0; s < nsteps; ++s) {
         if (step_enqueue(h, h.cur, ev) != 0) return GAM_ERR_CUDA;
-        h.cur ^= 1;
+        h.stepped();
         CK(cudaEventSynchronize(ev[NPHASE]));
         for (int q = 0; q < NPHASE; ++q) {
             float f = 0.f;
@@ -702,6 +702,7 @@ int gam_gpu_set_precision(gam_gpu_t* G, int mode) {
     if (mode != GAM_FP64 && mode != GAM_FP32FLUX) return GAM_ERR_ARG;
     if (mode == GAM_FP32FLUX && ensure_f32(G->h) != 0) return GAM_ERR_CUDA;
     if (mode != G->h.prec) {
+        half_planes(G->h, G->h.stream);
         G->h.prec = mode;
         destroy_graphs(G->h);
     }
@@ -725,15 +726,8 @@ int gam_gpu_fetch(gam_gpu_t* G, const char* name, double* out, long long n) {
     else if (s == "ogas") put(oS.gas, 5);
     else if (s == "omagflux") { put(oS.mf, 3); e = fe; }
     else if (s == "obxyz") put(oS.b, 3);
-    else if (s == "hgas") {
-        if (h.prec == PREC_FP64 && !h.p.doBoris) launch_half_con(h, h.stream);
-        put(h.H.gas, 5);
-    }
-    else if (s == "hmagflux") {
-        if (h.prec == PREC_FP64 && h.p.doMHD) launch_half_flux(h, h.stream);
-        put(h.H.mf, 3);
-        e = fe;
-    }
+    else if (s == "hgas") { half_planes(h, h.stream); put(h.H.gas, 5); }
+    else if (s == "hmagflux") { half_planes(h, h.stream); put(h.H.mf, 3); e = fe; }
     else if (s == "hbxyz") put(h.H.b, 3);
     else if (s == "efld") put(h.E, 3);
     else if (s == "vf") put(h.Vf, 3);
@@ -981,7 +975,7 @@ int ens_launch(gam_ensemble* E) {
     for (size_t m = 0; m < E->members.size(); ++m) {
         if (!E->active[m]) continue;
         Handle& h = E->members[m]->h;
-        h.cur ^= 1;
+        h.stepped();
         h.launches += kernels_per_step(h);
         if (E->queue) {   // its flux launches are the shared queue launches, counted on the first member
             h.launches -= h.p.do25D ? 2 : 3;

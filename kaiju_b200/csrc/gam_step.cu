@@ -922,17 +922,20 @@ void launch_min_length(Handle& h, cudaStream_t st) {
     h.launches++;
 }
 
-void launch_half_con(Handle& h, cudaStream_t st) {
-    PrimP Wh;
-    for (int v = 0; v < 5; ++v) Wh.w[v] = h.Wh[v];
-    k_half_con<<<grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB), TPB, 0, st>>>(h.L, h.p, Wh, h.H);
-    h.launches++;
-}
-
-void launch_half_flux(Handle& h, cudaStream_t st) {
-    k_half_flux<<<nblk(h.L.E, 256), 256, 0, st>>>(h.L.E, h.gridP(), Vec3P{{h.hbA[0], h.hbA[1], h.hbA[2]}},
-                                                  Vec3P{{h.H.mf[0], h.H.mf[1], h.H.mf[2]}});
-    h.launches++;
+void half_planes(Handle& h, cudaStream_t st) {
+    if (!h.halfDerived) return;
+    h.halfDerived = false;
+    if (!h.p.doBoris) {
+        PrimP Wh;
+        for (int v = 0; v < 5; ++v) Wh.w[v] = h.Wh[v];
+        k_half_con<<<grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB), TPB, 0, st>>>(h.L, h.p, Wh, h.H);
+        h.launches++;
+    }
+    if (h.p.doMHD) {
+        k_half_flux<<<nblk(h.L.E, 256), 256, 0, st>>>(h.L.E, h.gridP(), Vec3P{{h.hbA[0], h.hbA[1], h.hbA[2]}},
+                                                      Vec3P{{h.H.mf[0], h.H.mf[1], h.H.mf[2]}});
+        h.launches++;
+    }
 }
 
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st) {
@@ -1089,6 +1092,7 @@ constexpr long long BRANCH_CELLS = 100000;
 
 int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     cudaStream_t st = h.stream;
+    h.enqPrec = h.prec;
     int openRange = -1;
     auto mark = [&](int ph) {
         if (ev) cudaEventRecord(ev[ph], st);

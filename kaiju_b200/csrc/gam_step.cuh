@@ -91,6 +91,11 @@ struct Handle {
     GridP gridP() const;
     StateP cur_state() const { return S[cur]; }
     StateP old_state() const { return S[cur ^ 1]; }
+    // after every step. In double precision a step leaves the half state's fluxes, and without Boris its conserved gas,
+    // to be formed from the planes it does write (half_planes); halfDerived: H does not hold them yet.
+    bool halfDerived = false;
+    int enqPrec = PREC_FP64;   // precision of the step last enqueued or captured (an ensemble's graph outlives a change)
+    void stepped() { cur ^= 1; halfDerived = enqPrec == PREC_FP64; }
 };
 
 // Kernels beside one another in a captured step: between go(q) and back(), launches on st go to side branch q of the graph,
@@ -163,10 +168,9 @@ void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st);
 // states named (the other is known to be bFlux2Fld of its fluxes)
 void mark_b_given(Handle& h, cudaStream_t st);
 void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st);
-// h.H.gas from the half-state primitives, which the FP64 step without Boris does not write
-void launch_half_con(Handle& h, cudaStream_t st);
-// h.H.mf from the face fields, which the FP64 step does not write
-void launch_half_flux(Handle& h, cudaStream_t st);
+// h.H.mf and, without Boris, h.H.gas of the last step where it was one in double precision: from its face fields and
+// primitives. For inspection, and before a change of precision, whose steps write other planes.
+void half_planes(Handle& h, cudaStream_t st);
 // withB: ghost B copied with the gas (set-up); a step leaves it to the bFlux2Fld of the ghost cells that follows
 void launch_bcs(Handle& h, const StateP& s, cudaStream_t st, bool withB = true);
 void launch_calcdt(Handle& h, const StateP& s, int mode, cudaStream_t st);   // mode 0: in-step, 1: initial (no time advance)

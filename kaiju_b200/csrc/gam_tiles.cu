@@ -277,7 +277,7 @@ int tiles_launch(gam_tiles* T) {
         int rc = enqueue_tiled_step(T, 0);
         if (rc) return rc;
     }
-    for (size_t q = 0; q < T->t.size(); ++q) H(T, (int)q).cur ^= 1;
+    for (size_t q = 0; q < T->t.size(); ++q) H(T, (int)q).stepped();
     return GAM_OK;
 }
 
@@ -518,7 +518,7 @@ int gam_gpu_step_ghosts(gam_gpu_t* G) {
     Handle& h = capi_handle(G);
     if (h.tilePhase != 2) return GAM_ERR_ARG;
     step_enqueue_ghosts(h, h.cur);
-    h.cur ^= 1;
+    h.stepped();
     h.tilePhase = 0;
     int rc = capi_download_scalars(G);
     if (rc) return rc;

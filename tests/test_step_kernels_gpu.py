@@ -106,6 +106,29 @@ def test_side_by_side_equals_one_stream(gpu_lib, oracle_lib, kind, n):
 
 
 @pytest.mark.gpu
+def test_half_state_belongs_to_the_last_step(gpu_lib, oracle_lib):
+    """The half state of the last step stays what it is while the precision is changed: a change writes no half state, and
+    the planes of one mode do not stand for the other's step. (With FP32 fluxes the half state's gas is kept as floats for
+    the fluxes only, so that mode's is not fetched.)"""
+    from kaiju_b200 import gamera as gm
+    o, g = oracle_and_gpu("bw", (16, 16, 16))
+    with g:
+        o.step()
+        g.step()
+        for mode in (gm.GAM_FP32FLUX, gm.GAM_FP64):   # a step in double precision, first fetched after the change
+            g.set_precision(mode)
+            for name in ("hgas", "hmagflux"):
+                assert max(per_var_rel(g.fetch(name), o.get(name))) <= TOL, (mode, name)
+        g.set_precision(gm.GAM_FP32FLUX)
+        resync(o, g)
+        o.step()
+        g.step()   # a step with FP32 fluxes, whose face fluxes of the half state are still double
+        for mode in (gm.GAM_FP32FLUX, gm.GAM_FP64):
+            g.set_precision(mode)
+            assert max(per_var_rel(g.fetch("hmagflux"), o.get("hmagflux"))) <= TOL, mode
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["fp64", "fp32flux"])
 def test_given_cell_field(gpu_lib, oracle_lib, prec):
     """A Bxyz that is not bFlux2Fld of its fluxes (as a host may send) enters the limiter and the first step's old field
