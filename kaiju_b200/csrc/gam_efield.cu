@@ -14,7 +14,6 @@
 namespace gam {
 
 // ------------------------------------------------------------------ Mom2Face (fields.F90:235-285)
-struct Vec3F { float* v[3]; };
 // Vf at one face (explicit fused multiply-adds): the Central8 sums along dT1 of volume * velocity over that of the
 // volumes (clamped at TINY), each weight applied to its volume once for the four sums. A is the accumulation type:
 // double on the FP64 path, float on the FP32-flux path, whose velocities and volumes are float copies and whose Vf
@@ -43,8 +42,7 @@ __device__ __forceinline__ void mom2face_sum(const A* wV, const A* w0, const A* 
 // one another in the grid (blockIdx.y = slab), so the planes cross HBM about once. One face and direction at a time, 96
 // loads per cell, took 650 us at 256^3 (450 in single precision); now 484 (251).
 template <typename A> struct Vf9 { A* v[3][3]; };
-constexpr int M2F_TB = 128, SLAB = 8;
-template <typename A> constexpr int M2F_RUN = 8;
+constexpr int M2F_TB = 128, SLAB = 8, M2F_RUN = 8;
 // blocks per slab of each direction
 struct M2fGrid { int bI, bJ, bK, cI, cJ; };   // and 4-face chunks along i, RUN-face chunks along j
 
@@ -52,7 +50,7 @@ template <typename A>
 __global__ void __launch_bounds__(M2F_TB) k_mom2face3(Lay L, const A* __restrict__ vol, const A* __restrict__ v0,
                                                       const A* __restrict__ v1, const A* __restrict__ v2, Vf9<A> out,
                                                       Reg rI, Reg rJ, Reg rK, M2fGrid g) {
-    constexpr int RUN = M2F_RUN<A>;
+    constexpr int RUN = M2F_RUN;
     const int slab = blockIdx.y * SLAB;
     const A* const src[4] = {vol, v0, v1, v2};
     int b = blockIdx.x;
@@ -99,7 +97,7 @@ __global__ void __launch_bounds__(M2F_TB) k_mom2face3(Lay L, const A* __restrict
     }
     b -= g.bI;
     // a run of faces along j or k from the face at (i, f0): cells f0 - 4 .. f0 + RUN + 2
-    auto run = [&](const Reg& r, int first, int last, long long c, long long s, A* const* o) {
+    auto run = [&](int first, int last, long long c, long long s, A* const* o) {
         A w[4][RUN + 7];
 #pragma unroll
         for (int n = 0; n < RUN + 7; ++n)
@@ -121,7 +119,7 @@ __global__ void __launch_bounds__(M2F_TB) k_mom2face3(Lay L, const A* __restrict
         t /= rJ.ni;
         const int j = rJ.j0 + RUN * (t % g.cJ), k = rJ.k0 + slab + t / g.cJ;
         if (t / g.cJ >= SLAB || k >= rJ.k0 + rJ.nk) return;
-        run(rJ, j, rJ.j0 + rJ.nj - 1, L.at(i, j, k), L.P, out.v[0]);
+        run(j, rJ.j0 + rJ.nj - 1, L.at(i, j, k), L.P, out.v[0]);
         return;
     }
     b -= g.bJ;
@@ -131,14 +129,14 @@ __global__ void __launch_bounds__(M2F_TB) k_mom2face3(Lay L, const A* __restrict
         if (j >= rK.j0 + rK.nj) return;
         static_assert(SLAB % RUN == 0, "runs of a slab");
         for (int k = rK.k0 + slab; k < rK.k0 + slab + SLAB && k < rK.k0 + rK.nk; k += RUN)
-            run(rK, k, rK.k0 + rK.nk - 1, L.at(i, j, k), (long long)L.P * L.Q, out.v[1]);
+            run(k, rK.k0 + rK.nk - 1, L.at(i, j, k), (long long)L.P * L.Q, out.v[1]);
     }
 }
 
 template <typename A>
 static void launch_mom2face(const Lay& L, const A* vol, const A* v0, const A* v1, const A* v2, const Vf9<A>& out,
                             const Reg& rI, const Reg& rJ, const Reg& rK, cudaStream_t st) {
-    constexpr int RUN = M2F_RUN<A>;
+    constexpr int RUN = M2F_RUN;
     M2fGrid g;
     g.cI = (rI.ni + 3) / 4;
     g.cJ = (rJ.nj + RUN - 1) / RUN;
