@@ -72,23 +72,33 @@ __global__ void k_predict_faces(long long E, Par p, GridP g, Vec3P mf, Vec3P omf
 }
 
 // bFlux2Fld of the half-state face fluxes (Q + pdt (Q - oQ) / odt) of one cell, for the first steps after a state
-// came from outside (Scal::bGiven); out of line, so that the usual path keeps its registers
-__device__ __noinline__ void half_bxyz(const Lay& L, const GridP& g, const StateP& n, const StateP& o, double pdt,
-                                       double iodt, long long c, double* B) {
+// came from outside (Scal::bGiven); out of line and before the cell's other loads, so that the usual path keeps its
+// registers, and straight-line, so that its 34 loads are in flight together. As a loop over the faces behind those loads
+// it took the predictor phase of a 256^3 step from 1.01 to 1.63 ms (0.87 to 1.53 with FP32 fluxes), now to 1.36 (1.24);
+// always from the fluxes, with no field to extrapolate, the phase took 1.51 (1.29).
+struct V3 { double x, y, z; };
+__device__ __noinline__ V3 half_bxyz(const Lay& L, const GridP& g, const StateP& n, const StateP& o, double pdt,
+                                     double iodt, long long c) {
     const long long up[3] = {c + 1, c + L.P, c + (long long)L.P * L.Q};
-    const double idV = 1.0 / g.volume[c];
-    double lo[3], hi[3], Div = 0.0;
+    double q[6], oq[6];
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double q = n.mf[d][c], qu = n.mf[d][up[d]];
-        lo[d] = q + pdt * ((q - o.mf[d][c]) * iodt);
-        hi[d] = qu + pdt * ((qu - o.mf[d][up[d]]) * iodt);
-        Div += hi[d] - lo[d];
+        q[d] = n.mf[d][c]; q[3 + d] = n.mf[d][up[d]];
+        oq[d] = o.mf[d][c]; oq[3 + d] = o.mf[d][up[d]];
     }
+    const double idV = 1.0 / g.volume[c];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) q[f] = q[f] + pdt * ((q[f] - oq[f]) * iodt);
+    const double Div = q[3] - q[0] + q[4] - q[1] + q[5] - q[2];
+    double B[3];
+#pragma unroll
     for (int x = 0; x < 3; ++x) {
         double b = 0.0;
-        for (int d = 0; d < 3; ++d) b += hi[d] * g.xfc[d][x][up[d]] - lo[d] * g.xfc[d][x][c];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) b += q[3 + d] * g.xfc[d][x][up[d]] - q[d] * g.xfc[d][x][c];
         B[x] = (b - Div * g.xyzcc[x][c]) * idV;
     }
+    return V3{B[0], B[1], B[2]};
 }
 
 // bFlux2Fld of the half state + PredictCell (mhdgroup.F90:492-518, 529-563) on every cell, plus the
@@ -112,16 +122,18 @@ __global__ void k_predict_cells(const __grid_constant__ Lay L, const __grid_cons
     const StepTimes tm = step_times(sc);
     const double pdt = tm.pdt, iodt = tm.iodt;
     double Q[5], oQ[5], W[5], oW[5], pW[5], pQ[5], B[3] = {0.0, 0.0, 0.0}, nB[3];
+    const bool given = sc->bGiven > 0;
+    if (p.doMHD && given) {
+        const V3 b = half_bxyz(L, g, n, o, pdt, iodt, c);
+        B[0] = b.x; B[1] = b.y; B[2] = b.z;
+    }
 #pragma unroll
     for (int v = 0; v < 5; ++v) { Q[v] = n.gas[v][c]; oQ[v] = o.gas[v][c]; }
 #pragma unroll
     for (int x = 0; x < 3; ++x) nB[x] = n.b[x][c];
-    if (p.doMHD) {
-        if (sc->bGiven) half_bxyz(L, g, n, o, pdt, iodt, c, B);
-        else {
+    if (p.doMHD && !given) {
 #pragma unroll
-            for (int x = 0; x < 3; ++x) B[x] = nB[x] + pdt * ((nB[x] - o.b[x][c]) * iodt);
-        }
+        for (int x = 0; x < 3; ++x) B[x] = nB[x] + pdt * ((nB[x] - o.b[x][c]) * iodt);
     }
     cellC2P(p, oQ, oW);
     cellC2P(p, Q, W);
@@ -176,17 +188,33 @@ __global__ void k_half_flux(long long E, GridP g, Vec3P hbA, Vec3P hmf) {
 // bit, what a step leaves: bFlux2Fld of its fluxes, with the cells across the axis taking their conjugates'
 // (RingFlux2FieldFix). A restart's Bxyz is, so it goes on exactly as the run it was taken from.
 __global__ void k_b_given(Scal* sc, int steps) { sc->bGiven = steps; }
-__global__ void k_b_check(Lay L, Par p, GridP g, StateP s, int steps, Scal* sc) {
-    int i, j, k;
-    if (!reg_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, i, j, k)) return;
-    int jp = j, kp = k;
-    if (p.doRing && ((p.ringDoS && j < L.js()) || (p.ringDoE && j > L.je()))) lfmCC(L, p.ringDoS, p.ringDoE, j, k, jp, kp);
+// Both states in one pass over the metrics, by a grid that fits the GPU: a state that differs is known by the first cell
+// that does, and the threads then stop (one pass per state by a thread per cell took 0.9 ms of a 60 ms push at 256^3 with
+// equal fields and 0.8 with different ones, now 0.8, which is the traffic, and nothing).
+__device__ __forceinline__ bool b_differs(const Lay& L, const GridP& g, const StateP& s, long long c, long long src) {
     double B[3];
-    cellBxyz(L, g, s.mf, L.at(i, jp, kp), B);
-    const long long c = L.at(i, j, k);
+    cellBxyz(L, g, s.mf, src, B);
     bool same = true;
+#pragma unroll
     for (int x = 0; x < 3; ++x) same = same && __double_as_longlong(B[x]) == __double_as_longlong(s.b[x][c]);
-    if (!same && sc->bGiven < steps) atomicMax(&sc->bGiven, steps);
+    return !same;
+}
+__global__ void k_b_check(const __grid_constant__ Lay L, const __grid_constant__ Par p, const __grid_constant__ GridP g,
+                          const __grid_constant__ StateP n, const __grid_constant__ StateP o, bool doN, bool doO, Scal* sc) {
+    const unsigned cells = (unsigned)L.Ni * L.Nj;
+    volatile int* given = &sc->bGiven;
+    for (int k = blockIdx.y; k < L.Nk; k += gridDim.y)
+        for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < cells; t += gridDim.x * blockDim.x) {
+            if (*given >= (doN ? B_GIVEN_STEPS : 1)) return;
+            const int j = t / (unsigned)L.Ni, i = t - j * (unsigned)L.Ni;
+            int jp = j, kp = k;
+            if (p.doRing && ((p.ringDoS && j < L.js()) || (p.ringDoE && j > L.je())))
+                lfmCC(L, p.ringDoS, p.ringDoE, j, k, jp, kp);
+            const long long c = L.at(i, j, k), src = L.at(i, jp, kp);
+            const bool dn = doN && b_differs(L, g, n, c, src), dq = doO && b_differs(L, g, o, c, src);
+            if (dn) atomicMax(&sc->bGiven, B_GIVEN_STEPS);
+            else if (dq) atomicMax(&sc->bGiven, 1);
+        }
 }
 
 // Flux2Deltas (stress.F90:150-196); O is the flux storage type (float on the FP32-flux path), the sums
@@ -909,12 +937,12 @@ void mark_b_given(Handle& h, cudaStream_t st) {
     h.launches++;
 }
 void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st) {
-    const dim3 grid = grid_plane(Reg{0, h.L.Ni, 0, h.L.Nj, 0, h.L.Nk}, TPB);
     k_b_given<<<1, 1, 0, st>>>(h.dScal, 0);
     h.launches++;
-    if (!h.p.doMHD) return;   // no fluxes to follow
-    if (n) { k_b_check<<<grid, TPB, 0, st>>>(h.L, h.p, h.gridP(), h.S[h.cur], B_GIVEN_STEPS, h.dScal); h.launches++; }
-    if (o) { k_b_check<<<grid, TPB, 0, st>>>(h.L, h.p, h.gridP(), h.S[h.cur ^ 1], 1, h.dScal); h.launches++; }
+    if (!h.p.doMHD || !(n || o)) return;   // no fluxes to follow; nothing to look at
+    const unsigned ny = h.L.Nk < 64 ? h.L.Nk : 64, nx = std::min(nblk((long long)h.L.Ni * h.L.Nj, TPB), 37u);   // 16 per SM
+    k_b_check<<<dim3(nx, ny), TPB, 0, st>>>(h.L, h.p, h.gridP(), h.S[h.cur], h.S[h.cur ^ 1], n, o, h.dScal);
+    h.launches++;
 }
 
 void launch_min_length(Handle& h, cudaStream_t st) {

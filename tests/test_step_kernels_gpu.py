@@ -148,3 +148,22 @@ def test_given_cell_field(gpu_lib, oracle_lib, prec):
         tol = 1e-9 if prec == "fp64" else 2e-5   # three free-running steps; single-precision fluxes
         for name in STATE:
             assert max(per_var_rel(g.fetch(name), o.get(name))) <= tol, name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["bxyz", "obxyz"])
+@pytest.mark.parametrize("cell", [(4, 4, 4), (27, 11, 19), (9, 8, 12)])
+def test_given_field_of_one_cell(gpu_lib, oracle_lib, name, cell):
+    """One cell of one of the two states is enough for the half state's field to come from the fluxes."""
+    o, g = oracle_and_gpu("bw", (24, 8, 16))
+    o.step()
+    b = o.get(name)
+    b[cell] = (0.3, -0.2, 0.4)
+    o.set(name, b)
+    with g:
+        resync(o, g)
+        for _ in range(2):
+            o.step()
+            g.step()
+            for q in STATE:
+                assert max(per_var_rel(g.fetch(q), o.get(q))) <= TOL, q
