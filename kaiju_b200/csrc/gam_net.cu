@@ -268,6 +268,9 @@ struct DwShape {
     static constexpr int STAGE = 9 * XWIN + 3 * GWIN;
     static constexpr int NS = CINP == 32 ? 2 : 3;
     static constexpr int COLS = NG * 96 <= 256 ? 256 : 512;
+    // reading warps: four per group, one for the last, whose ninth window is 32 rows at most; MMA issue; copies
+    static constexpr int READERS = (NG - 1) * 128 + 32, THREADS = READERS + 64;
+    static_assert((NG - 1) * G == 8 && CINP <= 32, "the last group holds one window");
     // the last group's rows beyond the ninth window read what follows it (their results are not used)
     static constexpr int SLACK = NG * G * XWIN > STAGE ? NG * G * XWIN - STAGE : 0;
     static constexpr int BYTES = NS * STAGE + SLACK + 1024;
@@ -278,22 +281,31 @@ struct DwShape {
 // pair share x[c' + off(dj, dk)] and shift dy instead, so a tile of 128 cells c' takes 9 windows of x and 3 of dy, and
 // one MMA contracts 16 of its cells for 4 (or 8) windows' channels (M = 128) against 3 shifts x 32 output channels
 // (N = 96). Both operands are MN-major: the rows that a tensor copy brings in are the contraction index, and nothing is
-// transposed or copied by threads. A CTA accumulates all its tiles in TMEM and writes one partial; a fixed-order sum
-// follows. Cells outside [c0, c1) have a zero gradient, so the tiles need no masks.
-// Building A with 2-byte loads (one per element and tap) took 153 us per 32-channel layer at 32^3; now 17.3.
-template <int CINP>
-__global__ void __launch_bounds__(192, 1) k_conv_dw(const __grid_constant__ CUtensorMap xmap,
+// transposed or copied by threads. Cells outside [c0, c1) have a zero gradient, so the tiles need no masks.
+//
+// The tensor core truncates when it adds to an accumulator, so the error grows with the number of MMAs added one after
+// the other. The accumulators therefore take a chain of 8 at most, and the reading warps add the chains, rounded to
+// nearest, in registers (one row and 96 columns per thread); a CTA writes one partial for all its tiles and a fixed-order
+// sum in double follows. Boxes so small that two CTAs per SM, taking 16 cells at a time, would add fewer than 8 MMAs each
+// have a tile or two per CTA and few partials to sum: chains of 2 there (launch_dw). Against double sums of the same operands, 32-channel layers, 16^3 / 24^3 /
+// 32^3 / 40^3: 0.7 / 1.7 / 1.7 / 1.7e-7 (two CTAs per SM adding all they have: 0.9 / 1.7 / 3.1 / 5.1e-7, one: 1.6 / 3.3 /
+// 6.0 / 10e-7). The MMAs wait for the readers: a layer's gradient takes 2 to 3 us longer for it at 32^3.
+// Building A with 2-byte loads (one per element and tap) took 153 us per 32-channel layer at 32^3; now about 20.
+template <int CINP, int CHAIN>
+__global__ void __launch_bounds__(DwShape<CINP>::THREADS, 1) k_conv_dw(const __grid_constant__ CUtensorMap xmap,
                                                     const __grid_constant__ CUtensorMap gmap, DwArgs a) {
     using S = DwShape<CINP>;
     extern __shared__ unsigned char smraw[];
     unsigned char* sbase = align1k(smraw);
-    __shared__ __align__(8) uint64_t full[S::NS], empty[S::NS], done;
+    __shared__ __align__(8) uint64_t full[S::NS], empty[S::NS], ready, drained, last;
     __shared__ uint32_t tmemBase;
     __shared__ int failed;
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
         for (int q = 0; q < S::NS; ++q) { tc::mbar_init(&full[q], 1); tc::mbar_init(&empty[q], 1); }
-        tc::mbar_init(&done, 1);
+        tc::mbar_init(&ready, 1);
+        tc::mbar_init(&drained, S::READERS / 32);
+        tc::mbar_init(&last, 1);
         failed = 0;
         tma::fence_barrier_init();
     }
@@ -304,32 +316,40 @@ __global__ void __launch_bounds__(192, 1) k_conv_dw(const __grid_constant__ CUte
     const uint32_t tbase = tmemBase;
     const long long ntiles = (a.c1 - a.c0 + 2 + ROWS - 1) / ROWS;   // c' in [c0 - 1, c1 + 1)
     const long long myTiles = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    if (tid == 128) {
+    const long long chains = myTiles * (ROWS / 16 / CHAIN);
+    if (tid == S::READERS) {
+        // ---------------- MMA issue
         const uint32_t idesc = tc::idesc_bf16_f32_mn(128, 96);
         constexpr uint32_t SWZ = CINP == 32 ? tc::SWZ_64B : tc::SWZ_32B, XROW = CINP * 2;
         bool ok = true;
-        long long T = 0;
-        for (; T < myTiles; ++T) {
+        long long n = 0;   // chains
+        for (long long T = 0; T < myTiles && ok; ++T) {
             const int st = (int)(T % S::NS);
             if (!tc::mbar_wait(&full[st], (uint32_t)((T / S::NS) & 1), WAIT_LIMIT)) { ok = false; break; }
             tc::fence_after_sync();
             const uint32_t xw = tc::smem_u32(sbase + st * S::STAGE), gw = xw + 9 * S::XWIN;
-            for (int ks = 0; ks < ROWS / 16; ++ks) {
-                const uint64_t bd = tc::desc_swz(gw + ks * 16 * 64, S::GWIN, 8 * 64, tc::SWZ_64B);
+            for (int k0 = 0; k0 < ROWS / 16; k0 += CHAIN, ++n) {
+                if (n > 0 && !tc::mbar_wait(&drained, (uint32_t)((n - 1) & 1), WAIT_LIMIT)) { ok = false; break; }
+                tc::fence_after_sync();
+                for (int ks = k0; ks < k0 + CHAIN; ++ks) {
+                    const uint64_t bd = tc::desc_swz(gw + ks * 16 * 64, S::GWIN, 8 * 64, tc::SWZ_64B);
 #pragma unroll
-                for (int g = 0; g < S::NG; ++g)
-                    tc::mma_bf16(tbase + g * 96,
-                                 tc::desc_swz(xw + g * S::G * S::XWIN + ks * 16 * XROW, S::XWIN, 8 * XROW, SWZ), bd, idesc,
-                                 T > 0 || ks > 0);
+                    for (int g = 0; g < S::NG; ++g)
+                        tc::mma_bf16(tbase + g * 96,
+                                     tc::desc_swz(xw + g * S::G * S::XWIN + ks * 16 * XROW, S::XWIN, 8 * XROW, SWZ), bd,
+                                     idesc, ks > k0);
+                }
+                tc::mma_commit(&ready);
             }
-            tc::mma_commit(&empty[st]);
+            if (ok) tc::mma_commit(&empty[st]);
         }
-        if (ok) tc::mma_commit(&done);
-        else {
+        if (!ok) {   // the MMAs issued so far complete before the CTA gives its memory back
             failed = 1;
-            if (T > 0) tc::mbar_wait(&empty[(int)((T - 1) % S::NS)], (uint32_t)(((T - 1) / S::NS) & 1), WAIT_LIMIT);
+            tc::mma_commit(&last);
+            tc::mbar_wait(&last, 0u, WAIT_LIMIT);
         }
-    } else if (tid == 160) {
+    } else if (tid == S::READERS + 32) {
+        // ---------------- copies
         bool ok = true;
         long long T = 0;
         for (; T < myTiles; ++T) {
@@ -347,24 +367,37 @@ __global__ void __launch_bounds__(192, 1) k_conv_dw(const __grid_constant__ CUte
         if (!ok) failed = 1;
         for (long long q = T > S::NS ? T - S::NS : 0; q < T; ++q)
             tc::mbar_wait(&full[(int)(q % S::NS)], (uint32_t)((q / S::NS) & 1), WAIT_LIMIT);
-    } else if (warp < 4 && myTiles > 0) {
-        if (tc::mbar_wait(&done, 0u, WAIT_LIMIT)) {
-            tc::fence_after_sync();
-            float* part = a.partial + (long long)blockIdx.x * S::NG * 128 * 96;
-#pragma unroll 1
-            for (int q = 0; q < S::NG * 3; ++q) {
-                const int g = q / 3, b = q % 3;
-                float acc[32];
-                tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + g * 96 + b * 32, acc);
-                if (g * S::G + tid / CINP < 9 && tid % CINP < a.cin) {
-                    float4* row = reinterpret_cast<float4*>(part + ((long long)g * 128 + tid) * 96 + b * 32);
+    } else if (tid < S::READERS && myTiles > 0) {
+        // ---------------- row tid % 128 of group tid / 128
+        const int g = tid / 128, row = tid % 128;
+        const uint32_t src = tbase + ((uint32_t)((warp & 3) * 32) << 16) + g * 96;
+        float acc[96];
 #pragma unroll
-                    for (int n = 0; n < 8; ++n) row[n] = make_float4(acc[4 * n], acc[4 * n + 1], acc[4 * n + 2], acc[4 * n + 3]);
-                }
+        for (int q = 0; q < 96; ++q) acc[q] = 0.f;
+        bool ok = true;
+        for (long long n = 0; n < chains; ++n) {
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(&ready, (uint32_t)(n & 1), WAIT_LIMIT));
+            if (!ok) break;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                float v[32];
+                tc::tmem_ld32(src + b * 32, v);
+#pragma unroll
+                for (int q = 0; q < 32; ++q) acc[b * 32 + q] += v[q];
             }
             tc::fence_before_sync();
-        } else failed = 1;
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(&drained);
+        }
+        if (!ok) failed = 1;
+        else if (g * S::G + row / CINP < 9 && row % CINP < a.cin) {
+            float4* out = reinterpret_cast<float4*>(a.partial + (((long long)blockIdx.x * S::NG + g) * 128 + row) * 96);
+#pragma unroll
+            for (int q = 0; q < 24; ++q) out[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+        }
     }
+    tc::fence_before_sync();
     __syncthreads();
     if (tid == 0 && failed) atomicExch(a.err, 1);
     if (warp == 0) tc::tmem_free(tbase, S::COLS);
@@ -391,11 +424,12 @@ __global__ void __launch_bounds__(768) k_dw_reduce(const float* partial, int nbl
 
 // bias gradient: per-block partial sums of the gradient w.r.t. the pre-activation over the cell range, then a
 // fixed-order sum. A thread reads 8 channels of a cell at once (one channel after the other over the whole range,
-// 2 bytes at a time, took 27 us at 32^3, and the final sum by one thread per channel 19 us; now 5.6 and 4.0).
-__global__ void __launch_bounds__(256) k_bias_partial(const __nv_bfloat16* dy, long long c0, long long c1, float* part) {
-    __shared__ float red[8][32];
+// 2 bytes at a time, took 27 us at 32^3, and the final sum by one thread per channel 19 us; now about 6 and 4). The sums run
+// in double: a thread adds several cells.
+__global__ void __launch_bounds__(256) k_bias_partial(const __nv_bfloat16* dy, long long c0, long long c1, double* part) {
+    __shared__ double red[8][32];
     const int tid = threadIdx.x, q = tid & 3;
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    double s[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (long long c = c0 + blockIdx.x * 64LL + (tid >> 2); c < c1; c += gridDim.x * 64LL) {
         const uint4 u = *reinterpret_cast<const uint4*>(dy + c * NET_PITCH + q * 8);
         const uint32_t r[4] = {u.x, u.y, u.z, u.w};
@@ -413,12 +447,12 @@ __global__ void __launch_bounds__(256) k_bias_partial(const __nv_bfloat16* dy, l
     }
     __syncthreads();
     if (tid < 32) {
-        float t = 0.f;
+        double t = 0.0;
         for (int w = 0; w < 8; ++w) t += red[w][tid];
         part[blockIdx.x * 32 + tid] = t;
     }
 }
-__global__ void __launch_bounds__(1024) k_bias_reduce(const float* part, int nblk, int cout, float* gb) {
+__global__ void __launch_bounds__(1024) k_bias_reduce(const double* part, int nblk, int cout, float* gb) {
     __shared__ double red[32][33];
     const int co = threadIdx.x & 31, r = threadIdx.x >> 5;
     double s = 0.0;
@@ -501,8 +535,10 @@ int net_init() {
     set_smem(k_conv<32, MODE_HIDDEN>, ConvShape<32>::BYTES);
     set_smem(k_conv<32, MODE_OUT>, ConvShape<32>::BYTES);
     set_smem(k_conv<32, MODE_BWD>, ConvShape<32>::BYTES);
-    set_smem(k_conv_dw<16>, DwShape<16>::BYTES);
-    set_smem(k_conv_dw<32>, DwShape<32>::BYTES);
+    set_smem(k_conv_dw<16, 2>, DwShape<16>::BYTES);
+    set_smem(k_conv_dw<16, 8>, DwShape<16>::BYTES);
+    set_smem(k_conv_dw<32, 2>, DwShape<32>::BYTES);
+    set_smem(k_conv_dw<32, 8>, DwShape<32>::BYTES);
     sm_count();
     return (int)cudaGetLastError();
 }
@@ -573,7 +609,9 @@ static int launch_dw(const __nv_bfloat16* x, const __nv_bfloat16* dy, const DwAr
         return (int)cudaErrorInvalidValue;
     const long long ntiles = (a.c1 - a.c0 + 2 + ROWS - 1) / ROWS;
     const int grid = ntiles < nblk ? (int)ntiles : nblk;
-    k_conv_dw<CINP><<<grid, 192, S::BYTES, st>>>(xmap, gmap, a);
+    const long long spread = ntiles * (ROWS / 16) / (2 * sm_count());   // 16-cell MMAs per CTA, two CTAs per SM
+    if (spread >= 8) k_conv_dw<CINP, 8><<<grid, S::THREADS, S::BYTES, st>>>(xmap, gmap, a);
+    else k_conv_dw<CINP, 2><<<grid, S::THREADS, S::BYTES, st>>>(xmap, gmap, a);
     k_dw_reduce<CINP><<<9 * a.cin, 768, 0, st>>>(a.partial, grid, gW, a.cin, cout);
     return 0;
 }
@@ -592,8 +630,9 @@ int net_backward(const NetBox& b, __nv_bfloat16* const wbwd[NET_LAYERS], NetBuff
         int rc = l == 0 ? launch_dw<16>(nb.act[l], nb.grad[l], d, nblk, gW, s.cout[l], st)
                         : launch_dw<32>(nb.act[l], nb.grad[l], d, nblk, gW, s.cout[l], st);
         if (rc) return rc;
-        k_bias_partial<<<nblk, 256, 0, st>>>(nb.grad[l], b.c0, b.c1, nb.partial);
-        k_bias_reduce<<<1, 1024, 0, st>>>(nb.partial, nblk, s.cout[l], gW + 27LL * s.cout[l] * s.cin[l]);
+        double* bpart = reinterpret_cast<double*>(nb.partial);   // the weights' partials have been summed
+        k_bias_partial<<<nblk, 256, 0, st>>>(nb.grad[l], b.c0, b.c1, bpart);
+        k_bias_reduce<<<1, 1024, 0, st>>>(bpart, nblk, s.cout[l], gW + 27LL * s.cout[l] * s.cin[l]);
         if (l > 0) {   // gradient w.r.t. the previous layer's pre-activation: through this layer, then GELU'
             ConvArgs a{};
             a.gz = nb.pre[l - 1]; a.w = wbwd[l];

@@ -13,8 +13,8 @@
 // 128 cells x input channels (one tensor copy, swizzled) by the weights of the three taps di = -1, 0, +1 at once
 // (N = 96); the epilogue adds the three results of neighbouring rows. The weight gradient contracts over cells instead
 // (M = 128 rows of (window, input channel), N = 3 shifts x 32 output channels, K = 16 cells per MMA, both operands
-// MN-major), each CTA accumulating all taps in TMEM over its cells and writing one partial that a fixed-order
-// reduction sums.
+// MN-major), each CTA adding all taps over its cells (chains of MMAs in TMEM, the chains in registers) and writing one
+// partial that a fixed-order reduction sums.
 #pragma once
 #include <cuda_bf16.h>
 #include <cstdint>

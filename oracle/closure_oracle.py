@@ -61,6 +61,17 @@ def forward_graph(params, x, requires_grad=False):
     return h, layers
 
 
+def hidden_activations(params: np.ndarray, x: np.ndarray) -> np.ndarray:
+    """The last hidden layer's activations (rounded to BF16) of the cell at the middle of x, per channel."""
+    import torch
+    import torch.nn.functional as F
+    with torch.no_grad():
+        h = _bf16(_to_torch(x))
+        for W, b in unpack(params)[:-1]:
+            h = _bf16(F.gelu(F.conv3d(h, _bf16(W), b)))
+    return h[0, :, h.shape[2] // 2, h.shape[3] // 2, h.shape[4] // 2].numpy()
+
+
 def net_forward(params: np.ndarray, x: np.ndarray) -> np.ndarray:
     import torch
     with torch.no_grad():

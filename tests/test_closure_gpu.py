@@ -50,3 +50,34 @@ def test_gradients_match_oracle(shape):
             assert rel < 1.5e-2, (cin, cout, n, rel)
             o += n
     c.close()
+
+
+@pytest.mark.parametrize("shape", [(16, 16, 16), (32, 32, 32), (48, 40, 40)])
+def test_output_layer_gradient_sums(shape):
+    """The sums over cells of the output layer's weight and bias gradients, against double sums of the same values: with
+    zero weights below it its activations are the same everywhere. The tensor core truncates each addition to an
+    accumulator (half of 2^-23 on the mean); a chain of 8 positive terms of a size is off by the sum of k/8 * 2^-24
+    over k = 1..8, 2.7e-7, and the rounding of the result adds 2^-24 at most, whatever the number of cells."""
+    import torch
+    from kaiju_b200 import gamera as gm
+    from oracle import closure_oracle as co
+    c = gm.Closure(*shape, seed=2)
+    rng = np.random.default_rng(11)
+    p = np.zeros_like(c.params())
+    o = 0
+    for cin, cout in co.LAYERS[:3]:
+        o += 27 * cin * cout
+        p[o:o + cout] = rng.uniform(0.5, 2.0, cout)
+        o += cout
+    c.set_params(p)
+    x = np.zeros((shape[0] + 8, shape[1] + 8, shape[2] + 8, 8), np.float32)
+    act = np.asarray(co.hidden_activations(p, x[:9, :9, :9]), np.float64)   # one value per channel
+    # exact in BF16, over many exponents, so that no sum of the products is exact in 24 bits
+    gout = co._bf16(torch.from_numpy(np.exp(2.0 * rng.normal(size=shape + (gm.CLOSURE_OUT,))).astype(np.float32))).numpy()
+    g = c.backward_host(x, gout).astype(np.float64)[o:]
+    c.close()
+    s = gout.astype(np.float64).sum(axis=(0, 1, 2))
+    cin, cout = co.LAYERS[3]
+    for got, want in ((g[:27 * cin * cout], np.tile(np.outer(s, act).ravel(), 27)), (g[27 * cin * cout:], s)):
+        rel = np.linalg.norm(got - want) / np.linalg.norm(want)
+        assert rel <= 2.7e-7 + 2.0 ** -24, rel
