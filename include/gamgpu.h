@@ -331,6 +331,9 @@ void gam_tiles_destroy(gam_tiles_t* g);   /* the tiles are not destroyed */
  * where side 0 is the lower k neighbour, side 1 the upper, and the message packed for side s is the one
  * the neighbour there unpacks on side 1-s. Initial set-up: halo_pack/unpack with
  * GAM_HALO_STATE|GAM_HALO_OSTATE|GAM_HALO_BXYZ, then calcdt_local ; allreduce ; calcdt_finish.
+ * The words also carry whether a tile holds a Bxyz that is not bFlux2Fld of its fluxes, which decides how
+ * the half state's field is formed: after gam_gpu_sync_to_device each tile goes by its own arrays in the next
+ * step (the cells two tiles share then agree to rounding) and all of them by any tile's from then on.
  * Replaces: haloUpdate and updateMpiBCs (gamapp_mpi.F90:579-663, :694-794). */
 #define GAM_HALO_STATE 1u      /* State (between step_bcs and step_ghosts: the new state)            */
 #define GAM_HALO_OSTATE 2u     /* oState                                                             */

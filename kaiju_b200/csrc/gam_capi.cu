@@ -282,6 +282,7 @@ int download_scalars(gam_gpu* G) {
     Handle& h = G->h;
     CK(cudaMemcpyAsync(h.hScal, h.dScal, sizeof(Scal), cudaMemcpyDeviceToHost, h.stream));
     CK(cudaStreamSynchronize(h.stream));
+    h.scalStale = false;
     return GAM_OK;
 }
 
@@ -526,10 +527,12 @@ int gam_gpu_sync_to_host(gam_gpu_t* G, unsigned what, double* gas, double* magfl
 int gam_gpu_set_scalars(gam_gpu_t* G, double t, double dt, double dt0, int ts, double time, double otime) {
     if (!G) return GAM_ERR_ARG;
     Handle& h = G->h;
+    int rc = h.scalStale ? download_scalars(G) : GAM_OK;   // the others stay as they are on the device
+    if (rc) return rc;
     h.hScal->t = t; h.hScal->dt = dt; h.hScal->dt0 = dt0; h.hScal->ts = ts; h.hScal->time = time;
     h.hScal->otime = otime; h.hScal->dtMinBits = 0x7FF0000000000000ull; h.hScal->nanCount = 0;
     h.hScal->status = 0; h.hScal->sticky = 0; h.hScal->waitFail = 0u;
-    int rc = upload_scalars(G);
+    rc = upload_scalars(G);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h.stream));
     return GAM_OK;

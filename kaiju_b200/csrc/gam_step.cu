@@ -186,7 +186,8 @@ __global__ void k_half_flux(long long E, GridP g, Vec3P hbA, Vec3P hmf) {
 }
 // Scal::bGiven after a state came from outside: `steps`, raised by k_b_check for a state whose Bxyz is not, bit for
 // bit, what a step leaves: bFlux2Fld of its fluxes, with the cells across the axis taking their conjugates'
-// (RingFlux2FieldFix). A restart's Bxyz is, so it goes on exactly as the run it was taken from.
+// (RingFlux2FieldFix). A restart's Bxyz is, so it goes on exactly as the run it was taken from. Tiles take the largest of
+// theirs (gam_tiles.cu).
 __global__ void k_b_given(Scal* sc, int steps) { sc->bGiven = steps; }
 // Both states in one pass over the metrics, by a grid that fits the GPU: a state that differs is known by the first cell
 // that does, and the threads then stop (one pass per state by a thread per cell took 0.9 ms of a 60 ms push at 256^3 with
@@ -932,7 +933,6 @@ GridP Handle::gridP() const {
 static const int TPB = 128;
 
 void mark_b_given(Handle& h, cudaStream_t st) {
-    h.hScal->bGiven = B_GIVEN_STEPS;   // set_scalars uploads the host's copy
     k_b_given<<<1, 1, 0, st>>>(h.dScal, B_GIVEN_STEPS);
     h.launches++;
 }

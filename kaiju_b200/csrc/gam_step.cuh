@@ -91,6 +91,7 @@ struct Handle {
     GridP gridP() const;
     StateP cur_state() const { return S[cur]; }
     StateP old_state() const { return S[cur ^ 1]; }
+    bool scalStale = false;    // the device's scalars were changed without the host's copy of them (hScal)
     // after every step. In double precision a step leaves the half state's fluxes, and without Boris its conserved gas,
     // to be formed from the planes it does write (half_planes); halfDerived: H does not hold them yet.
     bool halfDerived = false;
@@ -165,7 +166,7 @@ enum { PH_PREDICT = 0, PH_EFIELD, PH_FLUXES, PH_DELTAS, PH_UPDATE, PH_DT, PH_BCS
 void launch_min_length(Handle& h, cudaStream_t st);   // Grid%di, dj, dk -> dl, after either changes
 void launch_bflux2fld(Handle& h, const StateP& s, cudaStream_t st);
 // Scal::bGiven after State n and/or oState came from outside the step: set to its most, or found by checking the
-// states named (the other is known to be bFlux2Fld of its fluxes)
+// states named (the other is known to be bFlux2Fld of its fluxes); on the device only
 void mark_b_given(Handle& h, cudaStream_t st);
 void launch_b_check(Handle& h, bool n, bool o, cudaStream_t st);
 // h.H.mf and, without Boris, h.H.gas of the last step where it was one in double precision: from its face fields and

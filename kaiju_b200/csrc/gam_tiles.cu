@@ -126,32 +126,43 @@ int halo_states(const Handle& h, unsigned what, StateP* out) {
     return n;
 }
 
+// The tiles' half states come from the same formula in every tile, or the cells and faces that two tiles share would
+// differ in the last place: Scal::bGiven is the largest of the tiles', agreed with their dt. The second word carries the
+// NaN count above it (without NaNs its largest is the largest of all tiles; with them the run has failed).
 __global__ void k_red_pack(Scal* sc, long long* words) {
     // both words order like their values as signed 64-bit integers, so a MIN reduction works on either
     words[0] = (long long)sc->dtMinBits;
-    words[1] = 0x7FFFFFFFFFFFFFFFll - (long long)sc->nanCount;
+    words[1] = 0x7FFFFFFFFFFFFFFFll - (((long long)sc->nanCount << 2) | sc->bGiven);
 }
 __global__ void k_red_unpack(Scal* sc, const long long* words) {
+    const long long w = 0x7FFFFFFFFFFFFFFFll - words[1];
     sc->dtMinBits = (unsigned long long)words[0];
-    sc->nanCount = (unsigned)(0x7FFFFFFFFFFFFFFFll - words[1]);
+    sc->nanCount = (unsigned)(w >> 2);
+    sc->bGiven = (int)(w & 3);
 }
+static_assert(B_GIVEN_STEPS <= 3, "two bits");
 __global__ void k_red_reset(Scal* sc) {
     sc->dtMinBits = 0x7FF0000000000000ull;
     sc->nanCount = 0u;
 }
 __global__ void k_tiles_set_otime(Scal* sc) { sc->otime = sc->time - sc->dt; }   // init.F90's oState%time
 
-// the tiles' CalcDT minimum and NaN count, written back to every tile (CalcDT_mpi)
+// the tiles' CalcDT minimum, NaN count and given field, written back to every tile (CalcDT_mpi)
 __global__ void k_tiles_dtmin(Scal* const* sc, int n) {
     if (threadIdx.x != 0) return;
     unsigned long long b = ~0ull;
     unsigned nan = 0u;
+    int given = 0;
     for (int q = 0; q < n; ++q) {
         unsigned long long v = sc[q]->dtMinBits;
         b = v < b ? v : b;
         nan += sc[q]->nanCount;
+        given = sc[q]->bGiven > given ? sc[q]->bGiven : given;
     }
-    for (int q = 0; q < n; ++q) { sc[q]->dtMinBits = b; sc[q]->nanCount = nan; }
+    for (int q = 0; q < n; ++q) { sc[q]->dtMinBits = b; sc[q]->nanCount = nan; sc[q]->bGiven = given; }
+}
+__global__ void k_tiles_given(Scal* const* sc, int n, int steps) {
+    for (int q = threadIdx.x; q < n; q += 32) sc[q]->bGiven = steps;
 }
 
 int status_of(int st) {
@@ -296,6 +307,23 @@ int tiles_collect(gam_tiles* T) {
     return worst;
 }
 
+// the tiles' Scal::bGiven before their next step: the largest of them. A push to a tile since the last one
+// (gam_gpu_sync_to_device) looked at that tile alone; its host copy of the scalars is the current one.
+int tiles_agree(gam_tiles* T) {
+    const int n = (int)T->t.size();
+    int most = 0, least = B_GIVEN_STEPS;
+    for (int q = 0; q < n; ++q) {
+        const int b = H(T, q).hScal->bGiven;
+        most = b > most ? b : most;
+        least = b < least ? b : least;
+    }
+    if (most == least) return GAM_OK;
+    cudaSetDevice(T->dev0);
+    k_tiles_given<<<1, 32, 0, T->root>>>(T->dScals, n, most);
+    for (int q = 0; q < n; ++q) H(T, q).hScal->bGiven = most;
+    return cudaGetLastError() == cudaSuccess ? GAM_OK : GAM_ERR_CUDA;
+}
+
 // kernels of one tiled step per tile: those of a step in its parts and the halo fill (and the tiles'
 // dt minimum, counted on tile 0)
 void count_launches(gam_tiles* T) {
@@ -377,7 +405,7 @@ int gam_tiles_create(gam_tiles_t** out, gam_gpu_t* const* tiles, int n, int peri
     fan(T, [&](int q) { enqueue_fill(T, q, 0, true, true); });
     fan(T, [&](int q) {
         Handle& h = H(T, q);
-        mark_b_given(h, h.stream);
+        launch_b_check(h, true, true, h.stream);
         k_red_reset<<<1, 1, 0, h.stream>>>(h.dScal);
         launch_calcdt_partial(h, h.S[h.cur], h.stream);
     });
@@ -395,6 +423,7 @@ int gam_tiles_create(gam_tiles_t** out, gam_gpu_t* const* tiles, int n, int peri
 
 int gam_tiles_run_steps(gam_tiles_t* T, int nsteps) {
     if (!T || nsteps < 0) return GAM_ERR_ARG;
+    { int rc = tiles_agree(T); if (rc) return rc; }
     for (int s = 0; s < nsteps; ++s) {
         int rc = tiles_launch(T);
         if (rc) return rc;
@@ -404,6 +433,7 @@ int gam_tiles_run_steps(gam_tiles_t* T, int nsteps) {
 
 int gam_tiles_run_steps_timed(gam_tiles_t* T, int nsteps, double* ms) {
     if (!T || nsteps < 0 || !ms) return GAM_ERR_ARG;
+    { int rc = tiles_agree(T); if (rc) return rc; }
     if (T->oneDevice && !T->graph[0]) { int rc = tiles_build(T); if (rc) return rc; }
     cudaSetDevice(T->dev0);
     cudaEvent_t e0, e1;
@@ -583,7 +613,8 @@ int gam_gpu_halo_unpack(gam_gpu_t* G, int side, unsigned what, const void* src) 
         }
     launch_chunks(h, tab, h.stream);
     // a step's own halo fill (State, before step_ghosts) is followed by the halo's bFlux2Fld; any other is not
-    if (h.tilePhase != 2 || what != GAM_HALO_STATE) mark_b_given(h, h.stream);
+    if (h.tilePhase == 0) { launch_b_check(h, true, true, h.stream); h.scalStale = true; }
+    else if (what != GAM_HALO_STATE) { mark_b_given(h, h.stream); h.scalStale = true; }
     return cudaGetLastError() == cudaSuccess ? GAM_OK : GAM_ERR_CUDA;
 }
 

@@ -152,6 +152,87 @@ def test_split_step_pieces_match_single_domain(name):
     assert L.gam_gpu_step_ghosts(tiles[0].h) == gm.GAM_ERR_ARG
 
 
+ARRAYS = ("gas", "magflux", "bxyz", "ogas", "omagflux", "obxyz")
+GRID = ("xyzcc", "xfc", "di", "dj", "dk", "volume", "face", "edge", "tf", "te", "teb", "xyz")
+
+
+def _restarted(tile):
+    """A new tile from what a restart keeps of this one, and what sets its scalars afterwards."""
+    from kaiju_b200 import gamera as gm
+    a, s = {n: tile.fetch(n) for n in ARRAYS}, tile.status()
+    t = gm.GameraGPU.from_arrays(tile.model, {n: tile.fetch(n) for n in GRID}, a["gas"], a["magflux"], a["ogas"],
+                                 a["omagflux"], s["time"], s["otime"], bxyz=a["bxyz"], obxyz=a["obxyz"])
+    return t, lambda: t.set_scalars(s["t"], s["dt"], s["dt0"], s["ts"], s["time"], s["otime"])
+
+
+def test_tile_group_restart_goes_on_exactly():
+    """Tiles taken to new ones by their State, oState, Bxyz and scalars go on bit for bit as the group they were taken from."""
+    from kaiju_b200 import gamera as gm, tiling as tl
+    m, xyz, ic = _case("bw")
+    tiles, _ = tl.make_tiles(m, xyz, 2, ic)
+    with gm.TileGroup(tiles) as grp:
+        grp.run_steps(5)
+        again, scal = zip(*[_restarted(t) for t in tiles])
+        with gm.TileGroup(again) as grp2:
+            for f in scal:
+                f()
+            grp2.run_steps(4)
+            grp.run_steps(4)
+            for t, u in zip(tiles, again):
+                for n in ("gas", "magflux", "bxyz"):
+                    assert np.array_equal(t.fetch(n), u.fetch(n)), n
+
+
+@pytest.mark.parametrize("split", [False, True])
+def test_tiles_agree_on_a_given_field(split):
+    """A push to one tile of a Bxyz that is not bFlux2Fld of its fluxes, in a cell that the other does not hold: the values
+    the two tiles share stay the same bits. (Split steps: from the step after next on, as the words carry it.)"""
+    import torch
+    from kaiju_b200 import gamera as gm, tiling as tl
+    m, xyz, ic = _case("bw")
+    tiles, sp = tl.make_tiles(m, xyz, 2, ic)
+    nk = sp[0][1]
+
+    def push():
+        a, s = {n: tiles[0].fetch(n) for n in ARRAYS}, tiles[0].status()
+        a["bxyz"][10, 9, 5] *= 1.01   # first active k layer but one
+        tiles[0].sync_to_device(time=s["time"], otime=s["otime"], **a)
+
+    def shared():   # the K interface fluxes at the boundary between the tiles: the upper's ks is the lower's ke + 1
+        lo, up = tiles
+        for n, first in (("gflx", 10), ("mflx", 6)):
+            a, b = lo.fetch(n)[G:-G, G:-G, G + nk], up.fetch(n)[G:-G, G:-G, G]
+            assert np.array_equal(a.reshape(a.shape[:2] + (-1,), order="F")[..., first:],
+                                  b.reshape(b.shape[:2] + (-1,), order="F")[..., first:]), n
+    if not split:
+        with gm.TileGroup(tiles) as grp:
+            grp.run_steps(4)
+            push()
+            for _ in range(3):
+                grp.run_steps(1)
+                shared()
+        return
+    words = [torch.zeros(2, dtype=torch.int64, device="cuda") for _ in tiles]
+    L = gm.load_library()
+    lo_up = [tl.neighbours(q, 2, False) for q in range(2)]
+    _exchange(tiles, gm.GAM_HALO_STATE | gm.GAM_HALO_OSTATE | gm.GAM_HALO_BXYZ, lo_up)
+    for t, w in zip(tiles, words):
+        assert L.gam_gpu_calcdt_local(t.h, w.data_ptr()) == 0
+    torch.cuda.synchronize()
+    red = torch.stack(words).min(dim=0).values
+    for t, w in zip(tiles, words):
+        w.copy_(red)
+        torch.cuda.synchronize()
+        assert L.gam_gpu_calcdt_finish(t.h, w.data_ptr()) == 0
+    for _ in range(3):
+        _split_step(tiles, words, lo_up)
+    push()
+    for n in range(3):
+        _split_step(tiles, words, lo_up)
+        if n > 0:
+            shared()
+
+
 def test_tile_arguments_are_checked():
     from kaiju_b200 import gamera as gm, tiling as tl
     m, xyz, ic = _case("bw")
