@@ -1004,11 +1004,12 @@ static void launch_bc_periodic(Handle& h, const StateP& n, const StateP& s, cuda
     h.launches++;
 }
 
-// CalcDT's own finalization saves a launch; the many blocks of a large grid pay more for counting one another (256^3:
-// 287 us against 268 and the launch's 4)
+// CalcDT's own finalization saves a launch; the many blocks of a large grid pay more for counting one another. The
+// phase in us, in one launch and in two: 128x128x4 13.2 / 15.3, 64^3 (1,188 blocks) 15.2 / 17.4, 96^3 (3,724) 30.2 / 29.7,
+// 128^3 51.3 / 50.2, 160^3 86.5 / 82.6, 256^3 314 / 296.
 static bool dt_in_one(const Handle& h) {
     const dim3 g = grid_plane(reg_dt(h.L, h.p), 256);
-    return g.x * g.y <= 8192u;
+    return g.x * g.y <= 2048u;
 }
 static void launch_calcdt_mode(Handle& h, const StateP& s, int finalize, cudaStream_t st) {
     const Lay& L = h.L;
@@ -1116,7 +1117,16 @@ int kernels_per_step(const Handle& h, bool split) {
 static const char* const kPhaseRange[NPHASE] = {"Predictor", "E-Field", "Fluxes", "Flux2Deltas", "Update", "DT",
                                                 "BCs"};   // BCs is pushed by step_enqueue_bcs
 
-constexpr long long BRANCH_CELLS = 100000;
+// Largest problem whose kernels run beside one another. us per step with and without it, double precision / FP32 fluxes:
+//   4 to 25 k cells     32x32x4 37 / 62, 64x64x1 43 / 60, 24^3 45 / 65, 41 / 54, 32x28x28 56 / 75, 44 / 57
+//   33 to 51 k          32^3 72 / 88, 47 / 62, 128x64x4 82 / 89, 57 / 66, 40x40x32 99 / 107, 67 / 72
+//   64 to 77 k          40^3 129 / 121, 80 / 84 (zero-gradient sides 138 / 125, 89 / 91), 128x128x4 138 / 135,
+//                       96x96x8 122 / 127, 93 / 90, 48x40x40 133 / 127, 86 / 88, magnetosphere 48x42x32 226 / 228, 189 / 186
+//   131 k               128x128x8 193 / 183, magnetosphere 48x42x64 315 / 322, 250 / 241
+//   2.5D                256x256x1 184 / 189, 146 / 150, 312x312x1 248 / 255, 196 / 199, 512x512x1 607 / 599
+//   with a closure      40^3 230 / 228, 182 / 199, 48^3 293 / 287, 243 / 250
+// The graphs of a step with branches take 0.6 ms longer to set up.
+static long long branch_cells(const Handle& h) { return h.p.do25D || h.closure ? 100000 : 60000; }
 
 int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     cudaStream_t st = h.stream;
@@ -1139,10 +1149,9 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     StateP nS = h.S[cur], oS = h.S[cur ^ 1];
     // The fluxes and the E field, and the two predictors, run beside one another where they are far from filling the GPU:
     // a step is a chain of dependent launches, and a small problem's step costs the length of that chain. Not in larger
-    // problems, which gain nothing and pay for the joins, and not where other problems' steps run beside this one.
-    // 4,096 cells 64 -> 39 us per step, 65,536 cells 144 -> 139 (212 -> 210 in 2.5D); with branches everywhere 1.2 M
-    // cells 1281 -> 1288, 256^3 +3% and a 24-member ensemble 2.23 -> 2.31 ms.
-    Branches br(st, ev == nullptr && h.alone && (long long)L.Nip * L.Njp * L.Nkp <= BRANCH_CELLS);
+    // problems, which gain nothing and pay for the joins (branch_cells), and not where other problems' steps run beside
+    // this one (a 24-member ensemble's 20 steps 2.23 -> 2.31 ms with branches).
+    Branches br(st, ev == nullptr && h.alone && (long long)L.Nip * L.Njp * L.Nkp <= branch_cells(h));
     const float* corr = nullptr;
     // what the update writes: everything, or, where k_bc_periodic writes all that lies further out, the active cells and
     // the layer around them that CalcDT reads

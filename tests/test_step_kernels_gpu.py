@@ -1,5 +1,5 @@
-"""The step's kernels at the sizes where their launch rules change and where a tile, a run of faces or a ghost layer ends
-early. Against the oracle the bound is the parity tests' 1e-10; variants that differ only in the launch give the same
+"""The step's kernels at the sizes where their launch rules change (side branches, CalcDT's end, rings and axis rows that
+meet) and where a tile, a run of faces or a ghost layer ends early. Against the oracle the bound is the parity tests' 1e-10; variants that differ only in the launch give the same
 bits. The periodic sides' index map is checked on the CPU too, against the three sweeps it stands for."""
 import numpy as np
 import pytest
@@ -95,7 +95,8 @@ def test_odd_sizes(gpu_lib, oracle_lib, n):
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind,n", [("ot", (32, 24, 4)), ("bw", (24, 16, 16)), ("ot", (40, 24, 1))])
 def test_side_by_side_equals_one_stream(gpu_lib, oracle_lib, kind, n):
-    """A small problem's step on its side streams and the phase-timed step on one stream: the same bits."""
+    """A small problem's step, captured with side branches, and the phase-timed step, one kernel after the other: the same
+    bits. (Whether the branches run at the same time shows in the step's time only.)"""
     o, a = oracle_and_gpu(kind, n)
     b = mirror_to_gpu(o, a.model)
     with a, b:
@@ -167,3 +168,54 @@ def test_given_field_of_one_cell(gpu_lib, oracle_lib, name, cell):
             g.step()
             for q in STATE:
                 assert max(per_var_rel(g.fetch(q), o.get(q))) <= TOL, q
+
+
+def _ot_device(n, **kw):
+    from kaiju_b200 import gamera as gm
+    m = gm.Model(*n, CFL=0.3, bc=(gm.GAM_BC_PERIODIC,) * 6, tFin=1.0e30, **kw)
+    return gm.GameraGPU.from_corners(m, gm.corners_uniform(m, (0.0, 1.0, 0.0, 1.0, 0.0, n[2] / n[0])), "OT2D")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(48, 40, 31), (48, 40, 32), (312, 320, 1), (320, 320, 1)])
+def test_either_side_of_the_branch_rule(gpu_lib, n):
+    """60,000 cells, 100,000 in 2.5D: captured steps and the same kernels one after the other give the same bits."""
+    with _ot_device(n) as a, _ot_device(n) as b:
+        a.run_steps(3)
+        b.profile_phases(3)
+        for name in STATE:
+            assert np.array_equal(a.fetch(name), b.fetch(name)), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(720, 720, 1), (728, 728, 1)])
+def test_either_side_of_the_dt_rule(gpu_lib, n):
+    """2,048 blocks: CalcDT over the active cells, its minimum taken in its own launch and in one more, against the dt of
+    the state that the step leaves."""
+    with _ot_device(n, dtActive=True) as g:
+        for _ in range(2):
+            dt, _, _ = g.step()
+            act = (slice(4, -4),) * 3
+            q, b = g.fetch("gas")[act], g.fetch("bxyz")[act]
+            dl = np.minimum(np.minimum(g.fetch("di"), g.fetch("dj")), g.fetch("dk"))[act]
+            v2 = (q[..., 1:4] ** 2).sum(-1) / q[..., 0] ** 2
+            P = (g.model.gamma - 1.0) * (q[..., 4] - 0.5 * q[..., 0] * v2)
+            fast = np.sqrt(g.model.gamma * P / q[..., 0] + (b ** 2).sum(-1) / q[..., 0])
+            want = 0.3 * (dl / (np.sqrt(v2) + fast)).min()
+            assert abs(dt - want) <= 1e-13 * want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,ring", [((16, 8, 32), dict(NumR=4, Nch=[8, 16, 32, 32])), ((16, 9, 32), dict(NumR=4, Nch=[8, 16, 32, 32])),
+                                    ((16, 4, 32), dict(NumR=1, Nch=[16]))])
+def test_rings_and_axis_rows_that_meet(gpu_lib, oracle_lib, n, ring):
+    """Both poles' rings in one launch only where they do not meet; and as few rows between the axes as the ghosts take.
+    (With fewer, the oracle's metrics and half state of the axis ghosts are not finite either.)"""
+    o, g = oracle_and_gpu("lfmbw", n, ring=ring)
+    with g:
+        for _ in range(2):
+            o.step()
+            g.step()
+            for name in STATE:
+                assert max(per_var_rel(g.fetch(name), o.get(name))) <= TOL, name
+            resync(o, g)
