@@ -752,17 +752,19 @@ int gam_closure_backward_host(gam_closure_t* C, const float* in, const float* go
 // ================================================================================ the closure in the step
 namespace gam {
 
-const float* closure_enqueue_corr(Handle& h, const StateP& nS, cudaStream_t st) {
+int closure_enqueue_corr(Handle& h, const StateP& nS, cudaStream_t st, const float** corr) {
     gam_closure* C = h.closure;
     const Lay& L = h.L;
     NormP n = norm_of(C);
     C->nb.act[0] = C->act0;
     k_closure_input<<<grid_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, 256), 256, 0, st>>>(L, h.p.gamma, nS, n, C->act0);
-    net_forward(C->box, C->wfwd, C->params, C->nb, false, C->err, st);
+    const int rc = net_forward(C->box, C->wfwd, C->params, C->nb, false, C->err, st);
+    if (rc) return rc;   // no step with corrections that were not evaluated
     k_closure_corr<<<grid_plane(Reg{L.is(), L.Nip + 1, L.js(), L.Njp + 1, L.ks(), L.Nkp + 1}, 256), 256, 0, st>>>(
         L, C->nb.out, n, C->geom, C->corr);
     h.launches += 2 + NET_LAYERS;
-    return C->corr;
+    *corr = C->corr;
+    return 0;
 }
 
 void closure_enqueue_check(Handle& h, const StateP& nS, cudaStream_t st) {

@@ -540,6 +540,7 @@ int net_init() {
     set_smem(k_conv_dw<32, 2>, DwShape<32>::BYTES);
     set_smem(k_conv_dw<32, 8>, DwShape<32>::BYTES);
     sm_count();
+    if (!tma::encoder()) return (int)cudaErrorNotSupported;   // the windows are tensor copies
     return (int)cudaGetLastError();
 }
 

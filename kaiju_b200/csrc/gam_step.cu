@@ -1165,7 +1165,7 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     // learned closure: face corrections from the net on State n, needed by Flux2Deltas
     if (h.closure && part == STEP_ALL) {
         br.go(SIDE_NET);
-        corr = closure_enqueue_corr(h, nS, st);
+        if (int rc = closure_enqueue_corr(h, nS, st, &corr)) return rc;
         br.back();
     }
     if (p.doMHD) {
@@ -1223,8 +1223,9 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     const bool fuse = h.fuseUpdate && !h.closure;
     // learned closure: a corrected update that fails positivity falls back to the plain fluxes (the second, conditional
     // Flux2Deltas). With the ensembles' tile queue the net runs here.
-    if (h.closure && !corr) corr = closure_enqueue_corr(h, nS, st);
-    else if (corr) br.join(SIDE_NET);
+    if (corr) br.join(SIDE_NET);
+    else if (h.closure)
+        if (int rc = closure_enqueue_corr(h, nS, st, &corr)) return rc;
     for (int pass = 0; pass < (fuse ? 0 : (corr ? 2 : 1)); ++pass) {
         const float* cq = pass == 0 ? corr : nullptr;
         const Scal* cond = pass == 0 ? nullptr : h.dScal;

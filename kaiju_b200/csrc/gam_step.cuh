@@ -179,7 +179,8 @@ double launch_divb(Handle& h, double* scratchDev, cudaStream_t st);
 int kernels_per_step(const Handle& h, bool split = false);   // split: as a tile's step is taken
 // learned closure in the step (gam_closure.cu): the net on State n and its face corrections (24 float
 // planes, area-scaled) before Flux2Deltas; after it the positivity check that sets Scal::closureReject
-const float* closure_enqueue_corr(Handle& h, const StateP& nS, cudaStream_t st);
+// (0 or a CUDA error code, as step_enqueue)
+int closure_enqueue_corr(Handle& h, const StateP& nS, cudaStream_t st, const float** corr);
 void closure_enqueue_check(Handle& h, const StateP& nS, cudaStream_t st);
 // the closure's EMF corrections added to the edge EMFs before E2Flux (skipped when the step fell back)
 void closure_enqueue_emf(Handle& h, cudaStream_t st);
