@@ -1162,8 +1162,8 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     const Reg act = {L.is(), L.Nip, L.js(), L.Njp, L.ks(), L.Nkp};
     if (part != STEP_POST) {
     mark(PH_PREDICT);
-    // learned closure: face corrections from the net on State n, needed by Flux2Deltas
-    if (h.closure && part == STEP_ALL) {
+    // learned closure: face corrections from the net on State n, needed by Flux2Deltas, whose phase they are timed with
+    if (h.closure && part == STEP_ALL && !ev) {
         br.go(SIDE_NET);
         if (int rc = closure_enqueue_corr(h, nS, st, &corr)) return rc;
         br.back();
@@ -1222,7 +1222,7 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     // without a closure the update computes the deltas itself (no dGasH/dGasM round trip through HBM)
     const bool fuse = h.fuseUpdate && !h.closure;
     // learned closure: a corrected update that fails positivity falls back to the plain fluxes (the second, conditional
-    // Flux2Deltas). With the ensembles' tile queue the net runs here.
+    // Flux2Deltas). With the ensembles' tile queue, and timed by phases, the net runs here.
     if (corr) br.join(SIDE_NET);
     else if (h.closure)
         if (int rc = closure_enqueue_corr(h, nS, st, &corr)) return rc;

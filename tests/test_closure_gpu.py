@@ -81,3 +81,18 @@ def test_output_layer_gradient_sums(shape):
     for got, want in ((g[:27 * cin * cout], np.tile(np.outer(s, act).ravel(), 27)), (g[27 * cin * cout:], s)):
         rel = np.linalg.norm(got - want) / np.linalg.norm(want)
         assert rel <= 2.7e-7 + 2.0 ** -24, rel
+
+
+def test_phase_times_count_the_network_with_the_deltas():
+    """profile_phases times the network with Flux2Deltas, which takes its corrections: many times the predictor's work."""
+    from kaiju_b200 import gamera as gm, turbulence as tu
+    g = tu.turbulence_problem(32, seed=5)
+    c = gm.Closure(32, 32, 32, seed=1)
+    plain = g.profile_phases(4)
+    g.set_closure(c)
+    g.profile_phases(2)
+    t = g.profile_phases(8)
+    assert t["predictor"] < 2.0 * plain["predictor"] + 0.02 and t["deltas"] > 2.0 * t["predictor"], (plain, t)
+    g.set_closure(None)
+    g.close()
+    c.close()
