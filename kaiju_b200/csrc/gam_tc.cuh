@@ -2,12 +2,13 @@
 // descriptors for kind::f16 (BF16 operands, FP32 accumulator), the MMA issue, its commit to an mbarrier,
 // bounded mbarrier waits and the TMEM -> register load of an accumulator.
 //
-// Operand layout used throughout: K-major, no swizzle. A matrix of R rows x K bf16 is a grid of "core
-// matrices" of 8 rows x 8 elements (8 x 16 bytes, rows 16 bytes apart, 128 contiguous bytes); core
-// matrices adjacent along K are LBO bytes apart, groups of 8 rows SBO bytes apart. For a row-block of
-// K = Kp elements stored K-chunk-minor: offset(r, k) = (r / 8) * (Kp / 8 * 128) + (k / 8) * 128 + (r % 8) * 16
-// + (k % 8) * 2, so LBO = 128 and SBO = Kp / 8 * 128; one MMA consumes K = 16 (two K chunks), and the
-// next K step starts 256 bytes further.
+// Operand layouts. The convolution's weights are K-major without swizzle: a matrix of R rows x K bf16 is a grid of "core
+// matrices" of 8 rows x 8 elements (8 x 16 bytes, rows 16 bytes apart, 128 contiguous bytes); core matrices adjacent
+// along K are LBO bytes apart, groups of 8 rows SBO bytes apart. For a row-block of K = Kp elements stored
+// K-chunk-minor: offset(r, k) = (r / 8) * (Kp / 8 * 128) + (k / 8) * 128 + (r % 8) * 16 + (k % 8) * 2, so LBO = 128 and
+// SBO = Kp / 8 * 128; one MMA consumes K = 16 (two K chunks), and the next K step starts 256 bytes further. Activations
+// and gradients are as tensor copies leave them, swizzled (desc_swz): K-major in the convolution, MN-major in its weight
+// gradient.
 #pragma once
 #include <cstdint>
 
@@ -69,8 +70,6 @@ __device__ __forceinline__ void mma_commit(uint64_t* mbar) {
 
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// generic-proxy shared-memory writes -> visible to the tensor core (async proxy)
-__device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(mbar)), "r"(count) : "memory");
