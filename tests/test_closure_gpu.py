@@ -52,6 +52,31 @@ def test_gradients_match_oracle(shape):
     c.close()
 
 
+def test_boxes_of_several_tiles_per_cta():
+    """A box in which every CTA of the convolution (two per SM, 126 cells a tile) takes three tiles or more, so that both
+    accumulators, the rows handed from warp to warp and the window ring come round again, and every CTA of the weight
+    gradient (one per SM, 128 cells) seven or eight, several turns of its ring. Forward and gradients against the oracle,
+    with the bounds of the small boxes."""
+    from kaiju_b200 import gamera as gm
+    from oracle import closure_oracle as co
+    shape = (40, 40, 40)   # 56 x 49 x 49 cells in the device's layout
+    c, p, x = _rand_case(shape, 13)
+    gout = np.random.default_rng(17).normal(size=shape + (gm.CLOSURE_OUT,)).astype(np.float32)
+    y, g = c.forward_host(x), c.backward_host(x, gout)
+    c.close()
+    ref = co.net_forward(p, x)
+    assert np.linalg.norm(y - ref) < 2e-3 * np.linalg.norm(ref)
+    # every cell by itself: one that took a wrong row for one of its 27 taps would be off by about 1 / sqrt(27) of the
+    # outputs' size, and a value on the other side of a BF16 rounding boundary moves one of its 864 terms by 2^-8 of it
+    assert np.abs(y - ref).max() < 0.05 * np.sqrt(np.mean(ref ** 2))
+    ref, o = co.net_grads(p, x, gout), 0
+    for cin, cout in co.LAYERS:
+        for n in (27 * cin * cout, cout):
+            rel = np.linalg.norm(g[o:o + n] - ref[o:o + n]) / np.linalg.norm(ref[o:o + n])
+            assert rel < 1.5e-2, (cin, cout, n, rel)
+            o += n
+
+
 @pytest.mark.parametrize("shape", [(16, 16, 16), (32, 32, 32), (48, 40, 40)])
 def test_output_layer_gradient_sums(shape):
     """The sums over cells of the output layer's weight and bias gradients, against double sums of the same values: with
