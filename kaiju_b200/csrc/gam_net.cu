@@ -68,8 +68,9 @@ __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" 
 // the epilogue adds out[c] = D[c-1][di=-1] + D[c][di=0] + D[c+1][di=+1] (a lane shuffle, and a row each side of a warp
 // through shared memory). The A operand is then read from shared memory once instead of three times -- with N = 32
 // that read, not the math, set the MMA's time -- and it needs no shifted start, so a window is a plain 128 x CINP box
-// that one tensor copy brings in swizzled, with no copy instructions in the other warps. What is left is the copies'
-// row rate: the 16- and the 32-channel layers, with half and twice the bytes and MMAs, take almost the same time.
+// that one tensor copy brings in swizzled, with no copy instructions in the other warps. No unit is near
+// its limit (32 channels, 64^3: math 21%, L2 27%, issue 45%); the 16- and the 32-channel layers, with half and twice the
+// bytes and MMAs, take almost the same time, so what is left goes with the nine windows of a tile, one after the other.
 // Warps 0-3: epilogue (warp w reads TMEM lanes 32w..32w+31). One thread of warp 4 issues the MMAs of a window once
 // full[s] completes, commits them to empty[s] and, after a tile's last window, to tfull[a]; one thread of warp 5 fills
 // the ring of NS windows. Two TMEM accumulators alternate; tempty[a] completes when the epilogue has read one.
