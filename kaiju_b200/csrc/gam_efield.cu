@@ -10,11 +10,29 @@
 //     areas and field; the 2x2 corner densities -- and evaluates GetCornerV, GetCornerD, GetCornerB (two
 //     limited EdgeLRs) and the EMF for its edge from shared memory.
 #include "gam_efield_tile.cuh"
-#include "gam_mom2face.cuh"
 
 namespace gam {
 
 // ------------------------------------------------------------------ Mom2Face (fields.F90:235-285)
+// Vf at one face (explicit fused multiply-adds): the Central8 sums along dT1 of volume * velocity over that of the
+// volumes (clamped at TINY), each weight applied to its volume once for the four sums. A is the accumulation type:
+// double on the FP64 path, float on the FP32-flux path, whose velocities and volumes are float copies and whose Vf
+// is stored as float.
+template <typename A>
+__device__ __forceinline__ void mom2face_sum(const A* wV, const A* w0, const A* w1, const A* w2, A& f0, A& f1, A& f2) {
+    A sV = A(0), s0 = A(0), s1 = A(0), s2 = A(0);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        A w = A(wC8(n)) * wV[n];
+        sV = sV + w;
+        s0 = fma(w, w0[n], s0);
+        s1 = fma(w, w1[n], s1);
+        s2 = fma(w, w2[n], s2);
+    }
+    const A idV = A(1) / (sV > A(TINY) ? sV : A(TINY));   // one reciprocal for the three quotients
+    f0 = s0 * idV; f1 = s1 * idV; f2 = s2 * idV;
+}
+
 // All three Mom2Face directions in one launch. out.v[eD]: the three component planes the edges of direction eD read
 // (dT1 = J, K, I for eD = I, J, K), written over the region of that direction.
 //
@@ -22,7 +40,7 @@ namespace gam {
 // keeps the window in registers: RUN faces along j (or k) read RUN + 7 cells each instead of 8 RUN, and 4 faces along i
 // are 12 cells in three 16- or 32-byte rows. The blocks of the three directions over the same SLAB k-planes stand next to
 // one another in the grid (blockIdx.y = slab), so the planes cross HBM about once. One face and direction at a time, 96
-// loads per cell, took 650 us at 256^3 (450 in single precision); now 484 (about 320, 67 of them for the differences).
+// loads per cell, took 650 us at 256^3 (450 in single precision); now 484 (251).
 template <typename A> struct Vf9 { A* v[3][3]; };
 constexpr int M2F_TB = 128, SLAB = 8, M2F_RUN = 8;
 // blocks per slab of each direction
