@@ -32,7 +32,7 @@ __device__ __forceinline__ StepTimes step_times(const Scal* sc) {
 // per-face values EdgeLRs divides out at every stencil point (fields.F90:335-336): flux/max(area,TINY)
 // for the half state (reconstruction) and for the limiting state.
 struct F32FaceOut { float* hbA[3]; float* nbA[3]; };
-struct F32CellOut { float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; };
+struct F32CellOut { float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; float* VdV[3]; };
 
 // Two consecutive face elements per thread with 16-byte loads and stores (E = P*Q*R is a multiple of 8 and
 // every plane starts 16-byte aligned), twice the bytes in flight per thread of a one-element loop; the
@@ -74,7 +74,7 @@ __global__ void k_predict_faces(long long E, Par p, GridP g, Vec3P mf, Vec3P omf
 // bFlux2Fld of the half-state face fluxes (Q + pdt (Q - oQ) / odt) of one cell, for the first steps after a state
 // came from outside (Scal::bGiven); out of line and before the cell's other loads, so that the usual path keeps its
 // registers, and straight-line, so that its 34 loads are in flight together. As a loop over the faces behind those loads
-// it took the predictor phase of a 256^3 step from 1.01 to 1.63 ms (0.87 to 1.53 with FP32 fluxes), now to 1.36 (1.24);
+// it took the predictor phase of a 256^3 step from 1.01 to 1.63 ms (0.94 to 1.58 with FP32 fluxes), now to 1.36 (1.29);
 // always from the fluxes, with no field to extrapolate, the phase took 1.51 (1.29).
 struct V3 { double x, y, z; };
 __device__ __noinline__ V3 half_bxyz(const Lay& L, const GridP& g, const StateP& n, const StateP& o, double pdt,
@@ -108,8 +108,9 @@ __device__ __noinline__ V3 half_bxyz(const Lay& L, const GridP& g, const StateP&
 // fluxes are Q + pdt (Q - oQ) / odt, so the half-state field is the same extrapolation of the two states' Bxyz: 6
 // values where the fluxes and their moment arms are 16. Mom2Face forms volume times velocity from the volumes and
 // the half-state primitives, and the corner densities are the half-state primitive density, so neither is written
-// here; the conserved half state is written only for the Boris fluxes (gam_gpu_fetch("hgas") rebuilds it from
-// the primitives). 448 B per zone before, about 232 now: 256^3 1.08 -> 0.68 ms, 0.92 -> 0.55 with FP32 fluxes.
+// here in double precision (with FP32 fluxes the products are, mom2face_sum says why); the conserved half state is
+// written only for the Boris fluxes (gam_gpu_fetch("hgas") rebuilds it from the primitives). 448 B per zone before, about
+// 232 now: 256^3 1.08 -> 0.68 ms, 0.92 -> 0.62 with FP32 fluxes (0.55 without the products).
 __global__ void k_predict_cells(const __grid_constant__ Lay L, const __grid_constant__ Par p,
                                 const __grid_constant__ GridP g, const __grid_constant__ StateP n,
                                 const __grid_constant__ StateP o, StateP h, PrimP Wh, PrimP Wn,
@@ -157,6 +158,9 @@ __global__ void k_predict_cells(const __grid_constant__ Lay L, const __grid_cons
         for (int v = 0; v < 5; ++v) f.Wn[v][c] = float(w[v]);
 #pragma unroll
         for (int x = 0; x < 3; ++x) { f.hb[x][c] = float(B[x]); f.nb[x][c] = float(nB[x]); }
+        const double V = g.volume[c] * (1.0 / dmax(pQ[0], p.dFloor));   // Mom2Face's summands (fields.F90:265-271)
+#pragma unroll
+        for (int x = 0; x < 3; ++x) f.VdV[x][c] = float(V * pQ[1 + x]);
         return;
     }
 #pragma unroll
@@ -1055,7 +1059,7 @@ void refresh_f32_background(Handle& h) {
 int ensure_f32(Handle& h) {
     if (h.f32pool) return 0;
     const long long E = h.L.E;
-    const int nplanes = 25 + 24 + 64 + 6 + (h.p.doBackground ? 18 : 0);   // 6: the I and J edges' face velocities
+    const int nplanes = 28 + 24 + 64 + 6 + (h.p.doBackground ? 18 : 0);   // 6: the I and J edges' face velocities
     if (cudaMalloc(&h.f32pool, sizeof(float) * E * nplanes) != cudaSuccess) return 3;
     cudaMemsetAsync(h.f32pool, 0, sizeof(float) * E * nplanes, h.stream);
     float* q = h.f32pool;
@@ -1069,6 +1073,7 @@ int ensure_f32(Handle& h) {
     for (int x = 0; x < 3; ++x) f.nbA[x] = take();
     for (int x = 0; x < 3; ++x) f.Vf[x] = take();
     for (int e = 0; e < 2; ++e) for (int x = 0; x < 3; ++x) f.VfE[e][x] = take();
+    for (int x = 0; x < 3; ++x) f.VdV[x] = take();
     for (int d = 0; d < 3; ++d) {
         for (int v = 0; v < 5; ++v) f.gflx[d][v] = take();
         for (int x = 0; x < 3; ++x) f.mflx[d][x] = take();
@@ -1185,7 +1190,7 @@ int step_enqueue(Handle& h, int cur, cudaEvent_t* ev, bool split, int part) {
     F32CellOut fc{};
     if (h.prec == PREC_FP32FLUX) {
         for (int v = 0; v < 5; ++v) { fc.Wh[v] = h.f32.Wh[v]; fc.Wn[v] = h.f32.Wn[v]; }
-        for (int x = 0; x < 3; ++x) { fc.hb[x] = h.f32.hb[x]; fc.nb[x] = h.f32.nb[x]; }
+        for (int x = 0; x < 3; ++x) { fc.hb[x] = h.f32.hb[x]; fc.nb[x] = h.f32.nb[x]; fc.VdV[x] = h.f32.VdV[x]; }
     }
     k_predict_cells<<<grid_plane(Reg{0, L.Ni, 0, L.Nj, 0, L.Nk}, TPB), TPB, 0, st>>>(L, p, g, nS, oS, h.H, Wh, Wn, fc, h.dScal);
     h.launches += 1;

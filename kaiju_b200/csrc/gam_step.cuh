@@ -15,6 +15,7 @@ enum Prec { PREC_FP64 = 0, PREC_FP32FLUX = 1 };
 // metric planes converted once
 struct F32Planes {
     float* Wh[5]; float* Wn[5]; float* hb[3]; float* nb[3]; float* hbA[3]; float* nbA[3]; float* Vf[3];
+    float* VdV[3];   // half-state volume * velocity, Mom2Face's summands
     float* VfE[2][3];   // face velocities for the I and J edges (Vf: the K edges')
     float* gflx[3][5]; float* mflx[3][3];   // area-scaled interface fluxes
     float* volume; float* face[3]; float* edge[3]; float* Tf[3][9]; float* Te[3][6]; float* Teb[3][4];

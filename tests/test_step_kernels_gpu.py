@@ -219,3 +219,24 @@ def test_rings_and_axis_rows_that_meet(gpu_lib, oracle_lib, n, ring):
             for name in STATE:
                 assert max(per_var_rel(g.fetch(name), o.get(name))) <= TOL, name
             resync(o, g)
+
+
+@pytest.mark.gpu
+def test_single_precision_e_field_error(gpu_lib):
+    """One step with FP32 fluxes and one without from the same state of the blast wave on the curvilinear grid: the E
+    field's relative root mean square difference. 2.610e-7 with Mom2Face's products volume * velocity formed in double and
+    rounded once (and in every build before they were dropped), 2.659e-7 with products of floats; the bound lies between."""
+    from kaiju_b200 import gamera as gm
+    m = gm.Model(64, 48, 40, CFL=0.3, bc=(gm.GAM_BC_ZEROGRAD,) * 6, tFin=1.0e30)
+    x = gm.corners_warped(m, (-0.5, 0.5) * 3, 0.04)
+    with gm.GameraGPU.from_corners(m, x, "BW") as g:
+        g.run_steps(25)
+        st, s, e = {q: g.fetch(q) for q in STATE + ("ogas", "omagflux", "obxyz")}, g.status(), []
+        for prec in (gm.GAM_FP64, gm.GAM_FP32FLUX):
+            with gm.GameraGPU.from_corners(m, x, "BW") as h:
+                h.set_precision(prec)
+                h.sync_to_device(time=s["time"], otime=s["otime"], **st)
+                h.set_scalars(s["t"], s["dt"], s["dt0"], s["ts"], s["time"], s["otime"])
+                h.step()
+                e.append(h.fetch("efld")[4:-4, 4:-4, 4:-4])
+    assert np.linalg.norm(e[1] - e[0]) <= 2.635e-7 * np.linalg.norm(e[0])
