@@ -308,11 +308,15 @@ int tiles_collect(gam_tiles* T) {
 }
 
 // the tiles' Scal::bGiven before their next step: the largest of them. A push to a tile since the last one
-// (gam_gpu_sync_to_device) looked at that tile alone; its host copy of the scalars is the current one.
+// (gam_gpu_sync_to_device) looked at that tile alone.
 int tiles_agree(gam_tiles* T) {
     const int n = (int)T->t.size();
     int most = 0, least = B_GIVEN_STEPS;
     for (int q = 0; q < n; ++q) {
+        if (H(T, q).scalStale) {
+            cudaSetDevice(H(T, q).device);
+            if (int rc = capi_download_scalars(T->t[q])) return rc;
+        }
         const int b = H(T, q).hScal->bGiven;
         most = b > most ? b : most;
         least = b < least ? b : least;
